@@ -37,31 +37,42 @@ static constexpr int UMMA_K = 16;
 static constexpr int W_TILE_BYTES = BM * BK * 2;  // 16 KiB
 static constexpr int SMEM_BUDGET = 200 * 1024;
 
-static constexpr int W_RAW_BYTES = BM * BK / 2;   // NVFP4: 128 rows x 32 bytes of packed e2m1 codes per k block
-static constexpr int W_SC_BYTES = BM * 16;        //        128 rows x 16 e4m3 block scales (4 k blocks of 64)
+// NVFP4: a raw stage holds 256 elements of K, 128 rows x 128 bytes of packed e2m1 codes (128-byte swizzle) and
+// 128 rows x 16 e4m3 block scales; it feeds four k blocks of 64
+static constexpr int W_RAW_BYTES = BM * 128;
+static constexpr int W_SC_BYTES = BM * 16;
+static constexpr int RAW_K = 256;
 
 template <int BN, bool DUAL, bool WFP4 = false, bool WFP8 = false>
 struct WgemmCfg {
   static constexpr int NW = DUAL ? 2 : 1;
   static constexpr int X_TILE_BYTES = BN * BK * 2;
   static constexpr int X_OFF = W_TILE_BYTES * NW;                 // operand tiles first (1024-byte aligned)
-  static constexpr int RAW_OFF = X_OFF + X_TILE_BYTES;            // NVFP4 only: packed codes, then block scales
-  static constexpr int SC_OFF = RAW_OFF + W_RAW_BYTES * NW;
-  static constexpr int STAGE_BYTES = WFP4 ? SC_OFF + W_SC_BYTES * NW : RAW_OFF;
-  static constexpr int THREADS = WFP4 ? 448 : 192;                // NVFP4 adds 8 de-quantisation warps
-  static constexpr int LUT_BYTES = WFP4 ? 512 : 0;                // e4m3 byte -> f16 table
+  // NVFP4: the stages hold activations only; the weights come through a ring of raw stages of their own and are
+  // expanded into tensor memory
+  static constexpr int STAGE_BYTES = WFP4 ? X_TILE_BYTES : X_OFF + X_TILE_BYTES;
+  static constexpr int THREADS = WFP4 ? 480 : 192;                // NVFP4 adds 8 de-quantisation warps and the producer
+                                                                  //   of the activations
   static constexpr int STAGES_RAW = SMEM_BUDGET / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 12 ? 12 : STAGES_RAW;
+  static constexpr int STAGES = WFP4 ? (BN <= 64 ? 8 : 4) : (STAGES_RAW > 12 ? 12 : STAGES_RAW);
+  static constexpr int ASTAGES = WFP4 ? 4 : 0;                    // expanded weight tiles in tensor memory
+  static constexpr int RAW_BYTES = NW * (W_RAW_BYTES + W_SC_BYTES);
+  static constexpr int RAW_FIT = (SMEM_BUDGET - STAGES * STAGE_BYTES) / RAW_BYTES;
+  static constexpr int RAWS = WFP4 ? (RAW_FIT > 6 ? 6 : RAW_FIT) : 0;
   static constexpr int ACC_COLS = BN * (DUAL ? 2 : 1);
-  // bf16 / NVFP4: two accumulators (one drains while the next tile runs). FP8: a ring of four PARTIAL accumulators,
-  // one per 128-wide k block, which the epilogue warps scale and add up in registers
-  static constexpr int NACC = WFP8 ? 4 : 2;
-  static constexpr int TMEM_COLS = NACC * ACC_COLS < 32 ? 32 : NACC * ACC_COLS;
+  static constexpr int A_COLS = WFP4 ? NW * BK / 2 : 0;           // expanded weight tile(s) of a stage, f16 pairs
+  // bf16 / NVFP4: two accumulators where they fit (one drains while the next tile runs). FP8: a ring of four PARTIAL
+  // accumulators, one per 128-wide k block, which the epilogue warps scale and add up in registers
+  static constexpr int NACC = WFP8 ? 4 : (2 * ACC_COLS + ASTAGES * A_COLS <= 512 ? 2 : 1);
+  static constexpr int A_COL0 = NACC * ACC_COLS;
+  static constexpr int COLS_USED = NACC * ACC_COLS + ASTAGES * A_COLS;
+  static constexpr int TMEM_COLS = COLS_USED <= 32 ? 32 : (COLS_USED <= 64 ? 64 : (COLS_USED <= 128 ? 128
+                                                                                  : (COLS_USED <= 256 ? 256 : 512)));
   static constexpr int EPI_BYTES = 32 * BM * 4;  // fp32 staging of 32 token columns
-  static constexpr int SMEM_BYTES =
-      STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + 512 /*barriers*/ + LUT_BYTES;
-  static_assert(TMEM_COLS <= 512, "accumulators do not fit TMEM");
-  static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0, "TMEM column count must be a power of two");
+  static constexpr int RING_BYTES = RAWS * RAW_BYTES + STAGES * STAGE_BYTES;
+  static constexpr int SMEM_BYTES = RING_BYTES + EPI_BYTES + 1024 /*align slack*/ + 512 /*barriers*/;
+  static_assert(!WFP4 || RAWS >= 2, "too few raw stages");
+  static_assert(COLS_USED <= 512, "accumulators do not fit TMEM");
 };
 
 struct WorkItem {
@@ -92,14 +103,12 @@ __device__ __forceinline__ bool decode_work(const WgemmArgs& a, int w, int n_tok
   return true;
 }
 
-// e4m3 (fn) byte -> f16 bits; every e4m3 value is exact in f16
-__device__ __forceinline__ uint32_t e4m3_f16_bits(uint32_t b) {
-  const uint32_t e = (b >> 3) & 15u, m = b & 7u;
-  float v;
-  if (e == 0u) v = float(m) * 0.001953125f;                     // subnormals: m * 2^-9
-  else if (e == 15u && m == 7u) v = 0.f;                         // NaN pattern: treated as 0
-  else v = __uint_as_float(((e + 120u) << 23) | (m << 20));
-  return uint32_t(__half_as_ushort(__float2half_rn(v))) | ((b & 0x80u) << 8);
+// four e4m3 (fn) bytes -> f16 pairs (hardware conversion; every e4m3 value is exact in f16), NaN patterns as 0
+__device__ __forceinline__ void e4m3x4_to_f16x2(uint32_t v, uint32_t (&o)[2]) {
+  v &= ~__vcmpeq4(v & 0x7f7f7f7fu, 0x7f7f7f7fu);
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\t"
+      "cvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
+      : "=r"(o[0]), "=r"(o[1]) : "r"(v));
 }
 // four bytes of e2m1 code pairs -> four f16x2 words (hardware conversion, exact)
 __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t pk, uint32_t (&o)[4]) {
@@ -116,6 +125,26 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t v) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// A operand (f16 pairs in 32-bit cells, row = lane) from tensor memory
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 __device__ __forceinline__ float gate_act(float v, int act) {
   if (act == 0) return v / (1.f + __expf(-v));
   return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
@@ -127,24 +156,26 @@ __device__ __forceinline__ float gate_act(float v, int act) {
 // costs them instruction fetches.
 enum : int { UN_NONE = 0, UN_XIELU = 1, UN_RELU2 = 2, UN_BIAS = 3 };
 template <int BN, bool DUAL, bool OUT_F32, bool WFP4, bool WFP8 = false, int UNARY = UN_NONE>
-__global__ void __launch_bounds__(WFP4 ? 448 : 192, 1)
+__global__ void __launch_bounds__(WFP4 ? 480 : 192, 1)
 wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
              const __grid_constant__ CUtensorMap tmS, const WgemmArgs a) {
   using Cfg = WgemmCfg<BN, DUAL, WFP4, WFP8>;
   constexpr int STAGES = Cfg::STAGES;
   constexpr int NACC = Cfg::NACC;
-  constexpr int KBE = WFP8 ? 128 : BK;     // elements per k block: one 128-byte swizzle row of e4m3 or bf16
+  // elements per k block: one 128-byte swizzle row of e4m3, bf16 or e2m1
+  constexpr int KBE = WFP8 ? 128 : (WFP4 ? RAW_K : BK);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* stage = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::EPI_BYTES);
+  float* stage = reinterpret_cast<float*>(smem + Cfg::RING_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::RING_BYTES + Cfg::EPI_BYTES);
   uint64_t* full = bars;                  // [STAGES]
   uint64_t* empty = bars + STAGES;        // [STAGES]
   uint64_t* tfull = bars + 2 * STAGES;    // [NACC]
   uint64_t* tempty = bars + 2 * STAGES + 4;  // [NACC]
-  uint64_t* wready = bars + 2 * STAGES + 8;  // [STAGES] NVFP4: operand tile of the stage has been expanded
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8 + (WFP4 ? STAGES : 0));
-  uint16_t* lut_sc = reinterpret_cast<uint16_t*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::EPI_BYTES + 512);
+  uint64_t* wready = bars + 2 * STAGES + 8;  // [STAGES] NVFP4: operand tiles of the stage have been expanded
+  uint64_t* rfull = wready + STAGES;         // [RAWS] NVFP4: codes and scales have landed
+  uint64_t* rempty = rfull + Cfg::RAWS;      // [RAWS]        and have been expanded
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8 + (WFP4 ? STAGES + 2 * Cfg::RAWS : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_flag = reinterpret_cast<int*>(tmem_slot + 2);
 
@@ -155,7 +186,11 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
-      if (WFP4) mbar_init(&wready[s], 256);
+      if (WFP4) mbar_init(&wready[s], 4);   // one arrive per warp of the group that expands the k block
+    }
+    for (int r = 0; r < Cfg::RAWS; ++r) {
+      mbar_init(&rfull[r], 1);
+      mbar_init(&rempty[r], 8);
     }
     for (int i = 0; i < NACC; ++i) {
       mbar_init(&tfull[i], 1);
@@ -167,10 +202,6 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
   if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
-  }
-  if (WFP4 && threadIdx.x >= 192) {      // conversion tables, built by the de-quantisation warps
-    const uint32_t b = threadIdx.x - 192;                       // 0..255
-    lut_sc[b] = uint16_t(e4m3_f16_bits(b));
   }
   tc_fence_before();
   __syncthreads();
@@ -248,8 +279,54 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (WFP4 && lane == 0) {
+      // codes and scales of 256 elements of K at a time: rows of 128 bytes for the memory system, and the loads run
+      // ahead of the k blocks by the whole raw ring
       tma_prefetch_desc(&tmW);
+      tma_prefetch_desc(&tmS);
+      int r = 0, issued = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      WorkItem it;
+      for (int w = blockIdx.x; ok && decode_work<BN>(a, w, n_tok_tiles, it); w += gridDim.x) {
+        const int kb0 = it.ks * kb_per_split;
+        const int kb1 = min(num_kb, kb0 + kb_per_split);
+        const int wrow = it.group * a.rows_per_group + it.feat0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(&rempty[r], ph ^ 1, abort_flag)) {
+            *abort_flag = 1;
+            atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY | SITE_GEMM);
+            ok = false;
+            break;
+          }
+          uint8_t* st = smem + r * Cfg::RAW_BYTES;
+          mbar_expect_tx(&rfull[r], Cfg::RAW_BYTES);
+#pragma unroll
+          for (int t = 0; t < Cfg::NW; ++t) {
+            tma_load_2d(st + t * W_RAW_BYTES, &tmW, &rfull[r], kb * (RAW_K / 2), wrow + t * a.dual_offset);
+            tma_load_2d(st + Cfg::NW * W_RAW_BYTES + t * W_SC_BYTES, &tmS, &rfull[r], kb * (RAW_K / 16),
+                        wrow + t * a.dual_offset);
+          }
+          ++issued;
+          if (++r == Cfg::RAWS) { r = 0; ph ^= 1; }
+        }
+      }
+      if (!ok) {
+        const int n = issued < Cfg::RAWS ? issued : Cfg::RAWS;
+        for (int i = 0; i < n; ++i) {
+          int ri = r - 1 - i;
+          uint32_t p = ph;
+          if (ri < 0) { ri += Cfg::RAWS; p ^= 1; }
+          const uint64_t t0 = globaltimer_ns();
+          while (!mbar_try_wait(&rfull[ri], p) && globaltimer_ns() - t0 < 2000000ull) {}
+        }
+      }
+    }
+  }
+  if (warp == (WFP4 ? 14 : 0)) {
+    // ------------------------------------------------------------------ TMA producer: NVFP4 activations, else both operands
+    if (lane == 0) {
+      if (!WFP4) tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       int s = 0;
       uint32_t ph = 0;
@@ -260,30 +337,21 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         const int kb0 = it.ks * kb_per_split;
         const int kb1 = min(num_kb, kb0 + kb_per_split);
         const int wrow = it.group * a.rows_per_group + it.feat0;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        constexpr int XPK = WFP4 ? RAW_K / BK : 1;        // activation tiles per k block
+        for (int kb = kb0 * XPK; kb < kb1 * XPK; ++kb) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) {
             *abort_flag = 1;
             atomicCAS(a.status, 0, ST_TIMEOUT_EMPTY | SITE_GEMM);
             ok = false;
             break;
           }
-          uint8_t* st = smem + s * Cfg::STAGE_BYTES;
-          if (WFP4) {
-            // packed codes of this k block; the block scales come 4 k blocks (16 bytes per row) at a time
-            const bool sc = (kb % 4 == 0) || kb == kb0;
-            mbar_expect_tx(&full[s], Cfg::X_TILE_BYTES + Cfg::NW * (W_RAW_BYTES + (sc ? W_SC_BYTES : 0)));
-            tma_load_2d(st + Cfg::RAW_OFF, &tmW, &full[s], kb * (BK / 2), wrow);
-            if (DUAL) tma_load_2d(st + Cfg::RAW_OFF + W_RAW_BYTES, &tmW, &full[s], kb * (BK / 2), wrow + a.dual_offset);
-            if (sc) {
-              tma_load_2d(st + Cfg::SC_OFF, &tmS, &full[s], (kb / 4) * 16, wrow);
-              if (DUAL) tma_load_2d(st + Cfg::SC_OFF + W_SC_BYTES, &tmS, &full[s], (kb / 4) * 16, wrow + a.dual_offset);
-            }
-          } else {
-            mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+          uint8_t* st = smem + Cfg::RAWS * Cfg::RAW_BYTES + s * Cfg::STAGE_BYTES;
+          mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+          if (!WFP4) {
             tma_load_2d(st, &tmW, &full[s], kb * KBE, wrow);
             if (DUAL) tma_load_2d(st + W_TILE_BYTES, &tmW, &full[s], kb * KBE, wrow + a.dual_offset);
           }
-          tma_load_2d(st + Cfg::X_OFF, &tmX, &full[s], it.group * a.x_group_col + kb * KBE, it.tok0);
+          tma_load_2d(st + (WFP4 ? 0 : Cfg::X_OFF), &tmX, &full[s], it.group * a.x_group_col + kb * (KBE / XPK), it.tok0);
           ++issued;
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -322,8 +390,36 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
           }
           tc_fence_after();
         }
+        if constexpr (WFP4) {
+          // the expanded weights of a k block of 64 are the A operand in tensor memory, the f16 activations B
+          const uint32_t d0 = tmem_base + acc * Cfg::ACC_COLS;
+          for (int kb = kb0 * (RAW_K / BK); kb < kb1 * (RAW_K / BK); ++kb) {
+            if (!mbar_wait(&wready[s], ph, abort_flag)) {
+              *abort_flag = 1;
+              atomicCAS(a.status, 0, ST_TIMEOUT_FULL | SITE_GEMM);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t at = tmem_base + Cfg::A_COL0 + (kb % (RAW_K / BK)) * Cfg::A_COLS;
+            const uint64_t dx = umma_desc_k_sw128(smem_u32(smem + Cfg::RAWS * Cfg::RAW_BYTES + s * Cfg::STAGE_BYTES));
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t koff = uint64_t(k * UMMA_K * 2 / 16);
+              const uint32_t accum = (kb > kb0 * (RAW_K / BK) || k > 0) ? 1u : 0u;
+              umma_f16_ts(d0, at + k * (UMMA_K / 2), dx + koff, idesc, accum);
+              if (DUAL) umma_f16_ts(d0 + BN, at + BK / 2 + k * (UMMA_K / 2), dx + koff, idesc, accum);
+            }
+            umma_commit(&empty[s]);
+            if (++s == STAGES) { s = 0; ph ^= 1; }
+          }
+          if (!ok) break;
+          umma_commit(&tfull[acc]);
+          if (++acc == NACC) { acc = 0; acc_ph ^= 1; }
+          continue;
+        }
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full[s], ph, abort_flag) || (WFP4 && !mbar_wait(&wready[s], ph, abort_flag))) {
+          if (!mbar_wait(&full[s], ph, abort_flag)) {
             *abort_flag = 1;
             atomicCAS(a.status, 0, ST_TIMEOUT_FULL | SITE_GEMM);
             ok = false;
@@ -368,84 +464,101 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         }
       }
     }
-  } else if (WFP4 && warp >= 6) {
+  } else if (WFP4 && warp >= 6 && warp < 14) {
     // ------------------------------------------------------------------ NVFP4 de-quantisation (warps 6..13)
-    // The 256 threads expand every weight tile of a stage (128 rows x 64 codes) into the bf16, 128-byte-swizzled
-    // operand tile the MMA reads. A task is one 16-byte chunk (8 codes = 4 packed bytes): lane -> (row, chunk)
-    // such that a warp reads 128 contiguous bytes of codes and writes four complete 128-byte rows, so neither
-    // side has a shared-memory bank conflict. Codes become f16 pairs with the hardware conversion
-    // (cvt.rn.f16x2.e2m1x2) and are multiplied by the block scale as f16x2 (exact: 1 + 3 mantissa bits, range
-    // 2^-10 .. 2688); the MMA of this variant runs on f16 operands, so the bf16 activation tile of the stage is
-    // converted in place as well (clamped to the f16 range).
-    const int d = threadIdx.x - 192;
-    const int dw = d >> 5, dl = d & 31;
-    const int chunk = dl & 7;
-    const int row0 = dw * 4 + (dl >> 3);           // rows row0 + 32 * i, i = 0..3
-    int s = 0;
-    uint32_t ph = 0;
+    // Two groups of four warps take turns at the k blocks of 64. A thread owns one weight row (= lane of tensor memory):
+    // two 16-byte reads give its 64 codes (the 128-byte swizzle of the load puts eight rows of a column of chunks into
+    // eight different bank groups), the hardware conversion (cvt.rn.f16x2.e2m1x2) makes f16 pairs of them, a product with the
+    // block scale in f16x2 follows (exact: 1 + 3 mantissa bits, range 2^-10 .. 2688), and the row goes to tensor memory as
+    // A operand. The multiplication runs on f16, so the activation tile of the k block is converted in place as well
+    // (clamped to the f16 range).
+    // Bound by what a k block moves through shared memory and by the conversions: expanded tiles that pass through shared
+    // memory instead (written, then read by the tensor cores) and loads of 32 bytes a row, a k block of codes at a time,
+    // took 446 us for the gate and up rows of 512 experts (2 x 512 x 2048, 2170 rows of tokens) and 294 us for the
+    // rows behind, this 241 and 189.
+    const int grp = (warp - 6) >> 2;
+    const int q = warp & 3;                        // TMEM lane quarter this warp may write
+    const int row = q * 32 + lane;
+    const int d = threadIdx.x - 192 - grp * 128;   // thread of the group
+    int s = grp, r = 0, n = grp;                   // n: k block of this CTA, counted through its work items
+    uint32_t ph = 0, rph = 0;
     bool ok = true;
-    uint32_t scw[Cfg::NW][4][4];                   // [tile][row i][k block within the group of 4]: 4 scale bytes
-#pragma unroll
-    for (int t = 0; t < Cfg::NW; ++t)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) scw[t][i][k] = 0u;
     WorkItem it;
     for (int w = blockIdx.x; decode_work<BN>(a, w, n_tok_tiles, it); w += gridDim.x) {
       const int kb0 = it.ks * kb_per_split;
       const int kb1 = min(num_kb, kb0 + kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (ok && !mbar_wait(&full[s], ph, abort_flag)) {
+        if (ok && !__all_sync(0xffffffffu, mbar_wait(&rfull[r], rph, abort_flag))) {
           *abort_flag = 1;
           atomicCAS(a.status, 0, ST_TIMEOUT_FULL | SITE_GEMM);
-          ok = false;      // keep arriving so that nobody is left waiting on wready
+          ok = false;      // keep arriving so that nobody is left waiting
         }
-        uint8_t* st = smem + s * Cfg::STAGE_BYTES;
-        if (ok) {
-          const bool new_sc = (kb % 4 == 0) || kb == kb0;
-          const int kq = kb & 3;
+        const uint8_t* raw = smem + r * Cfg::RAW_BYTES;
 #pragma unroll
-          for (int t = 0; t < Cfg::NW; ++t) {
+        for (int i = 0; i < 2; ++i) {
+          const int kq = grp + 2 * i;              // k block of 64 within the raw stage
+          // the tile in tensor memory is free once the products of the k block that had it last are done: their
+          // activations' stage says so, which is not used again before this k block has been multiplied
+          const int o = n - Cfg::ASTAGES;
+          if (ok && !__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort_flag) &&
+                                                 (o < 0 || mbar_wait(&empty[o % STAGES], uint32_t(o / STAGES) & 1u, abort_flag)))) {
+            *abort_flag = 1;
+            atomicCAS(a.status, 0, ST_TIMEOUT_FULL | SITE_GEMM);
+            ok = false;
+          }
+          if (ok) {
+            tc_fence_after();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int row = row0 + 32 * i;
-              if (new_sc) {
-                const uint4 v = *reinterpret_cast<const uint4*>(st + Cfg::SC_OFF + t * W_SC_BYTES + row * 16);
-                scw[t][i][0] = v.x; scw[t][i][1] = v.y; scw[t][i][2] = v.z; scw[t][i][3] = v.w;
+            for (int t = 0; t < Cfg::NW; ++t) {
+              const uint8_t* codes = raw + t * W_RAW_BYTES + row * 128;
+              uint32_t sc[2];                      // scales of the row's four blocks of 16 codes
+              e4m3x4_to_f16x2(*reinterpret_cast<const uint32_t*>(raw + Cfg::NW * W_RAW_BYTES + t * W_SC_BYTES + row * 16 + kq * 4),
+                              sc);
+              const uint32_t at = tmem_base + (uint32_t(q * 32) << 16) + Cfg::A_COL0 + kq * Cfg::A_COLS + t * (BK / 2);
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const uint4 v = *reinterpret_cast<const uint4*>(codes + (((kq * 2 + h) ^ (row & 7)) * 16));
+                const uint32_t pk[4] = {v.x, v.y, v.z, v.w};
+                uint32_t o[16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                  const uint32_t sc2 = __byte_perm(sc[h], 0, c < 2 ? 0x1010 : 0x3232);
+                  uint32_t e[4];
+                  e2m1x8_to_f16x2(pk[c], e);
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    const __half2 p = __hmul2(*reinterpret_cast<const __half2*>(&e[j]),
+                                              *reinterpret_cast<const __half2*>(&sc2));
+                    o[c * 4 + j] = *reinterpret_cast<const uint32_t*>(&p);
+                  }
+                }
+                tmem_st16(at + h * 16, o);
               }
-              const uint32_t sw = kq == 0 ? scw[t][i][0] : (kq == 1 ? scw[t][i][1] : (kq == 2 ? scw[t][i][2] : scw[t][i][3]));
-              const uint32_t sb = lut_sc[(sw >> (8 * (chunk >> 1))) & 0xFFu];     // scale of this chunk's 16 block
-              const uint32_t sc2 = sb | (sb << 16);
-              const uint32_t pk = *reinterpret_cast<const uint32_t*>(st + Cfg::RAW_OFF + t * W_RAW_BYTES + row * 32 + chunk * 4);
-              uint32_t o[4];
-              e2m1x8_to_f16x2(pk, o);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&o[j]),
-                                          *reinterpret_cast<const __half2*>(&sc2));
-                o[j] = *reinterpret_cast<const uint32_t*>(&r);
-              }
-              *reinterpret_cast<uint4*>(st + t * W_TILE_BYTES + row * 128 + ((chunk ^ (row & 7)) * 16)) =
-                  make_uint4(o[0], o[1], o[2], o[3]);
             }
-          }
-          // the activations arrive as bf16: convert the X tile in place (chunk positions are unchanged)
-          uint4* xt = reinterpret_cast<uint4*>(st + Cfg::X_OFF);
+            uint4* xt = reinterpret_cast<uint4*>(smem + Cfg::RAWS * Cfg::RAW_BYTES + s * Cfg::STAGE_BYTES);
 #pragma unroll
-          for (int idx = d; idx < BN * 8; idx += 256) {
-            uint4 v = xt[idx];
-            v.x = bf16x2_to_f16x2(v.x); v.y = bf16x2_to_f16x2(v.y);
-            v.z = bf16x2_to_f16x2(v.z); v.w = bf16x2_to_f16x2(v.w);
-            xt[idx] = v;
+            for (int idx = d; idx < BN * 8; idx += 128) {
+              uint4 v = xt[idx];
+              v.x = bf16x2_to_f16x2(v.x); v.y = bf16x2_to_f16x2(v.y);
+              v.z = bf16x2_to_f16x2(v.z); v.w = bf16x2_to_f16x2(v.w);
+              xt[idx] = v;
+            }
+            tmem_st_wait();
+            fence_proxy_async_smem();
+            tc_fence_before();
           }
-          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&wready[s]);
+          s += 2;
+          n += 2;
+          if (s >= STAGES) { s -= STAGES; ph ^= 1; }
         }
-        mbar_arrive(&wready[s]);
-        if (++s == STAGES) { s = 0; ph ^= 1; }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&rempty[r]);
+        if (++r == Cfg::RAWS) { r = 0; rph ^= 1; }
       }
     }
-  } else {
+  } else if (warp >= 2 && warp < 6) {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     int acc = 0;
@@ -918,7 +1031,7 @@ int wgemm_launch(const WgemmHost& h, cudaStream_t stream) {
     return 1;
   }
   // NVFP4: h.w = packed codes [rows, K / 2] bytes (row pitch h.ldw bytes), h.w_scales = e4m3 [rows, K / 16]
-  const CUtensorMap* tmW = fp4 ? tmap_2d(h.w, uint64_t(h.w_rows), uint64_t(h.K / 2), uint64_t(h.ldw), BM, BK / 2, TM_U8, false)
+  const CUtensorMap* tmW = fp4 ? tmap_2d(h.w, uint64_t(h.w_rows), uint64_t(h.K / 2), uint64_t(h.ldw), BM, 128, TM_U8, true)
                            : fp8 ? tmap_2d(h.w, uint64_t(h.w_rows), uint64_t(h.K), uint64_t(h.ldw), BM, 128, TM_U8, true)
                                : tmap_2d(h.w, uint64_t(h.w_rows), uint64_t(h.K), uint64_t(h.ldw) * 2, BM, BK, TM_BF16, true);
   const CUtensorMap* tmS = fp4 ? tmap_2d(h.w_scales, uint64_t(h.w_rows), uint64_t(h.K / 16), uint64_t(h.K / 16), BM, 16,
@@ -976,7 +1089,7 @@ int wgemm_launch(const WgemmHost& h, cudaStream_t stream) {
     snprintf(g_gemm_err, sizeof(g_gemm_err), "wgemm: biases come with ungrouped bf16 gate/up weights and bf16 output");
     return 1;
   }
-  const int num_kb = fp8 ? h.K / 128 : (h.K + BK - 1) / BK;
+  const int num_kb = fp8 ? h.K / 128 : (fp4 ? h.K / RAW_K : (h.K + BK - 1) / BK);
   if (a.split_k > num_kb) a.split_k = num_kb;
   while (a.split_k > 1 && (a.split_k - 1) * ((num_kb + a.split_k - 1) / a.split_k) >= num_kb) --a.split_k;
   if (a.split_k > 1 && (!a.ws || !a.counters)) {
