@@ -433,10 +433,10 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // Rotate-half pairing (i, i + 32); cos_sin rows are [cos(32) | sin(32)].
 __global__ void __launch_bounds__(128)
 mla_prep_kernel(const __nv_bfloat16* __restrict__ kva, long ld_kva, const float* __restrict__ norm_w, float eps,
-                float w_offset, const __nv_bfloat16* __restrict__ q, long ld_q_tok, int q_head_stride, int q_pe_off,
+                float w_offset, const __nv_bfloat16* q, long ld_q_tok, int q_head_stride, int q_pe_off,
                 int nh, const float* __restrict__ cos_sin, const int* __restrict__ positions,
                 const long* __restrict__ slots, __nv_bfloat16* __restrict__ cache, long cell_stride,
-                __nv_bfloat16* __restrict__ q_abs) {
+                __nv_bfloat16* q_out, int q_out_row) {
   __shared__ float red[4];
   const int t = blockIdx.x, tid = threadIdx.x;
   const __nv_bfloat16* row = kva + long(t) * ld_kva;
@@ -471,7 +471,7 @@ mla_prep_kernel(const __nv_bfloat16* __restrict__ kva, long ld_kva, const float*
     const __nv_bfloat16* qp = q + long(t) * ld_q_tok + long(h) * q_head_stride + q_pe_off;
     const float a = __bfloat162float(qp[i]), b = __bfloat162float(qp[32 + i]);
     const float c = cs[i], sn = cs[32 + i];
-    __nv_bfloat16* qo = q_abs + (long(t) * nh + h) * MLA_DK + MLA_L;
+    __nv_bfloat16* qo = q_out + (long(t) * nh + h + 1) * q_out_row - MLA_R;      // (may be the columns just read)
     qo[i] = __float2bfloat16(a * c - b * sn);
     qo[32 + i] = __float2bfloat16(b * c + a * sn);
   }
@@ -502,13 +502,13 @@ int mla_start(const CUtensorMap& tq, const CUtensorMap& tc, const MlaArgs& a, di
 
 int mla_prep_launch(const void* kva, long ld_kva, const float* norm_w, float eps, float w_offset, const void* q,
                     long ld_q_tok, int q_head_stride, int q_pe_off, int nh, const float* cos_sin,
-                    const int* positions, const long* slots, void* cache, long cell_stride, void* q_abs, int T,
-                    cudaStream_t s) {
+                    const int* positions, const long* slots, void* cache, long cell_stride, void* q_out, int q_out_row,
+                    int T, cudaStream_t s) {
   if (T <= 0) return 0;
   mla_prep_kernel<<<T, 128, 0, s>>>(static_cast<const __nv_bfloat16*>(kva), ld_kva, norm_w, eps, w_offset,
                                     static_cast<const __nv_bfloat16*>(q), ld_q_tok, q_head_stride, q_pe_off, nh,
                                     cos_sin, positions, slots, static_cast<__nv_bfloat16*>(cache), cell_stride,
-                                    static_cast<__nv_bfloat16*>(q_abs));
+                                    static_cast<__nv_bfloat16*>(q_out), q_out_row);
   return cudaGetLastError() != cudaSuccess ? 1 : 0;
 }
 

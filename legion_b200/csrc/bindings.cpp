@@ -496,13 +496,15 @@ void mla_prep(const Tensor& kva, const Tensor& norm_w, double eps, double w_offs
               "mla_prep: cos_sin must be float32 [positions, 64]");
   TORCH_CHECK(positions.scalar_type() == at::kInt && slots.scalar_type() == at::kLong, "positions i32, slots i64");
   TORCH_CHECK(cache.is_contiguous() && cache.size(-1) == 576, "mla_prep: cache rows must be [.., 576]");
-  TORCH_CHECK(q_abs.is_contiguous() && q_abs.size(0) == q.size(0) && q_abs.size(1) == q.size(1) && q_abs.size(2) == 576,
-              "mla_prep: q_abs must be [T, heads, 576]");
+  TORCH_CHECK(q_abs.is_contiguous() && q_abs.size(0) == q.size(0) && q_abs.size(1) == q.size(1) &&
+                  (q_abs.size(2) == 576 || (q_abs.data_ptr() == q.data_ptr() && q_abs.size(2) == q_pe_off + 64)),
+              "mla_prep: q_abs must be [T, heads, 576] or q itself");
   c10::cuda::CUDAGuard guard(kva.device());
   TORCH_CHECK(lb::mla_prep_launch(kva.data_ptr(), kva.stride(0), norm_w.data_ptr<float>(), float(eps), float(w_offset),
                                   q.data_ptr(), q.stride(0), int(q.stride(1)), int(q_pe_off), int(q.size(1)),
                                   cos_sin.data_ptr<float>(), positions.data_ptr<int>(), slots.data_ptr<long>(),
-                                  cache.data_ptr(), 576, q_abs.data_ptr(), int(kva.size(0)), cur_stream()) == 0,
+                                  cache.data_ptr(), 576, q_abs.data_ptr(), int(q_abs.size(2)), int(kva.size(0)),
+                                  cur_stream()) == 0,
               "mla_prep launch failed");
 }
 

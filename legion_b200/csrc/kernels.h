@@ -54,8 +54,8 @@ int mla_attn_launch(const void* q_abs, long q_pitch, long T, const void* cache, 
 const char* mla_attn_last_error();
 int mla_prep_launch(const void* kva, long ld_kva, const float* norm_w, float eps, float w_offset, const void* q,
                     long ld_q_tok, int q_head_stride, int q_pe_off, int nh, const float* cos_sin,
-                    const int* positions, const long* slots, void* cache, long cell_stride, void* q_abs, int T,
-                    cudaStream_t s);
+                    const int* positions, const long* slots, void* cache, long cell_stride, void* q_out, int q_out_row,
+                    int T, cudaStream_t s);
 
 int router_topk_launch(const float* logits, long ldl, const float* bias, int E, int k, int mode, int renorm,
                        float route_scale, int n_group, int topk_group, int group_top, int* ids, float* wts,

@@ -628,23 +628,63 @@ class Decoder:
         wkv_b = w[f"{p}.mla.kv_b"].view(nh, dn + dvh, L)
         if x.is_cuda and x.dtype == torch.bfloat16 and ops.sm100.mla_supported(nh, L, dr, kv.page):
             # absorbed form on the tensor cores: q_abs = [q_nope W_uk | rope(q_pe)], o = (softmax . c_kv) W_uv
-            q_abs = torch.empty(T, nh, L + dr, dtype=x.dtype, device=x.device)
             own = (ops.sm100.TUNE["mla_head_gemm"] and dn % 64 == 0 and dvh % 8 == 0 and (dn + dr) % 8 == 0
                    and isinstance(w[f"{p}.mla.kv_b"], torch.Tensor))
+            if own and b.max_q_len >= ops.sm100.LATENT_EXPAND_MIN:
+                parts = ops.sm100.latent_parts(b, kv.page)
+                if ops.sm100.mla_expand_ok(q, w[f"{p}.mla.kv_b"], kv.k[il], parts[0], nh, dn, dr, dvh, L):
+                    return self._mla_parts(p, il, q, kva, b, kv, parts)
+            q_abs = torch.empty(T, nh, L + dr, dtype=x.dtype, device=x.device)
             if own:
                 # per-head absorb and value projections on the grouped tcgen05 GEMM (group = head), each head's
                 # slice read and written in place
-                uk = self._mla_uk.get(p)
-                if uk is None:
-                    uk = wkv_b[:, :dn].transpose(1, 2).contiguous().view(nh * L, dn)     # W_uk^T per head, K-major
-                    self._mla_uk[p] = uk
-                ops.sm100.head_linear(q.view(T, nh * (dn + dr)), uk, nh, L, L, dn, dn + dr, q_abs.view(T * nh, L + dr))
+                ops.sm100.head_linear(q.view(T, nh * (dn + dr)), self._absorb_rows(p, wkv_b), nh, L, L, dn, dn + dr,
+                                      q_abs.view(T * nh, L + dr))
             else:
                 q_abs[..., :L] = torch.bmm(q[..., :dn].transpose(0, 1), wkv_b[:, :dn]).transpose(0, 1)
             ops.sm100.mla_prep(kva, w[f"{p}.mla.kv_a_norm"], cfg.rms_eps, cfg.norm_offset, q, dn, self.cos_sin,
                                b.positions, b.slots, kv.k[il], q_abs)
             return self._mla_tail(p, il, q_abs, b, kv, own)
         return self._mla_reference(p, il, x, q, kva, b, kv)
+
+    def _absorb_rows(self, p: str, wkv_b):
+        """W_uk^T of every head, K-major: [heads * kv_lora, nope]."""
+        uk = self._mla_uk.get(p)
+        if uk is None:
+            dn = self.cfg.qk_nope_dim
+            uk = self._mla_uk[p] = wkv_b[:, :dn].transpose(1, 2).contiguous().view(-1, dn)
+        return uk
+
+    def _mla_parts(self, p: str, il: int, q, kva, b: StepBatch, kv: KvCache, parts):
+        """Latent attention of a step with long portions: those attend over keys and values of every head
+        (``ops.sm100.mla_prompt``), the other sequences in the latent space."""
+        cfg, w = self.cfg, self.w
+        T, nh = q.shape[0], q.shape[1]
+        L, dn, dr, dvh = cfg.kv_lora, cfg.qk_nope_dim, cfg.qk_rope_dim, cfg.v_head_dim
+        kv_b, scale = w[f"{p}.mla.kv_b"], cfg.attn_scale or (dn + dr) ** -0.5
+        ops.sm100.mla_prep(kva, w[f"{p}.mla.kv_a_norm"], cfg.rms_eps, cfg.norm_offset, q, dn, self.cos_sin, b.positions, b.slots,
+                           kv.k[il], q)
+        out = None
+        for part in parts:
+            qp = q if part.rows is None else q.index_select(0, part.rows)
+            n = qp.shape[0]
+            if part.expand:
+                o = ops.sm100.mla_prompt(qp, kv_b, kv.k[il], part, scale, nh, dn, dr, L)
+            else:
+                q_abs = torch.empty(n, nh, L + dr, dtype=q.dtype, device=q.device)
+                ops.sm100.head_linear(qp.view(n, nh * (dn + dr)), self._absorb_rows(p, kv_b.view(nh, dn + dvh, L)), nh, L, L, dn,
+                                      dn + dr, q_abs.view(n * nh, L + dr))
+                q_abs[..., L:].copy_(qp[..., dn:])
+                o_lat = ops.sm100.mla_attn(q_abs, kv.k[il], part.cu_q, part.ctx_lens, part.block_table, kv.page, part.max_q_len,
+                                           scale, max_ctx=part.max_ctx or None)
+                o = torch.empty(n, nh * dvh, dtype=q.dtype, device=q.device)
+                ops.sm100.head_linear(o_lat.view(n, nh * L), kv_b[dn:], nh, dn + dvh, dvh, L, L, o.view(n * nh, dvh))
+            if part.rows is None:
+                out = o
+            else:
+                out = torch.empty(T, nh * dvh, dtype=q.dtype, device=q.device) if out is None else out
+                out.index_copy_(0, part.rows, o)
+        return ops.linear(out, w[f"{p}.mla.o"])
 
     def _mla_tail(self, p: str, il: int, q_abs, b: StepBatch, kv: KvCache, own: bool):
         """Latent attention over the absorbed query rows, the per-head value projection and the output projection."""

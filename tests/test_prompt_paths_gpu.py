@@ -39,3 +39,30 @@ def test_moe_dequantised_prompt(T, E, k, H, F):
     # one bf16 rounding of the output, of the pair rows and (of a value near a tie) of the activations: 3 * 2^-9
     err = (out - want).norm() / want.norm()
     assert err < 3 * 2.0 ** -9, err
+
+
+# a long portion alone, behind cached tokens, beside short portions and a decode row; sizes around the pages of 64
+@pytest.mark.parametrize("lens,cached", [([192], 0), ([257, 3], 64), ([200, 1, 320], 37)])
+def test_latent_prompt_per_head_form(lens, cached, monkeypatch):
+    from legion_b200.config import ModelConfig
+    from legion_b200.engine.lm import EngineConfig, build_engine
+    from legion_b200.models.weights import random_weights
+    cfg = ModelConfig(arch="deepseek_v3", n_layer=2, hidden=256, vocab=512, n_head=4, n_kv_head=4, head_dim=192, kv_lora=512,
+                      qk_nope_dim=128, qk_rope_dim=64, v_head_dim=128, qk_norm=False, dense_ff=512)
+    w = random_weights(cfg, DEV, torch.bfloat16, seed=0, std=0.05)
+    out = []
+    for least in (192, 1 << 30):                    # the per-head form, then everything in the latent space
+        monkeypatch.setattr(sm(), "LATENT_EXPAND_MIN", least)
+        eng = build_engine(cfg, weights=dict(w), device=DEV, engine_cfg=EngineConfig(
+            ctx_size=1024, max_seqs=4, block_size=64, prefill_chunk=1024, max_batch_tokens=1024, prefix_cache=False), start=False)
+        toks = [torch.randint(0, 512, (n + cached,), generator=torch.Generator().manual_seed(n)).tolist() for n in lens]
+        seqs = [eng.open_sequence(str(i)) for i in range(len(lens))]
+        if cached:
+            eng.feed([(s, t[:cached], []) for s, t in zip(seqs, toks)])
+        logits = eng.feed([(s, t[cached:], [n - 1]) for s, t, n in zip(seqs, toks, lens)])
+        out.append((logits.double().cpu(), [k.double().cpu() for k in eng.kv.k.values()]))
+        eng.shutdown()
+    (a, ka), (b, kb) = out
+    # two orders of bf16 roundings (keys and values against queries and attended latents), two layers
+    assert (a - b).norm() < 0.01 * b.norm(), (a - b).norm() / b.norm()
+    assert torch.equal(ka[0], kb[0]) and (ka[1] - kb[1]).norm() < 0.01 * kb[1].norm()
