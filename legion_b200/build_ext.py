@@ -60,7 +60,7 @@ def _run(cmd: list[str]) -> str:
 # those every model launches, and those of its layer kinds. The binding files name all kernels; the subset is linked and
 # loaded with lazy binding, so the absent ones do not matter until something calls them.
 CORE_TARGET = ROOT / "_C_core.so"
-CORE = {"gemm_sm100", "sgemm", "elementwise", "sampling", "spec", "tmap", "logits", "bindings", "bindings_layers"}
+CORE = {"gemm_sm100", "gemm_pair_sm100", "sgemm", "elementwise", "sampling", "spec", "tmap", "logits", "bindings", "bindings_layers"}
 _ATTN = {"attn_prefill_sm100", "attn_decode_sm100", "attn_decode", "attn_general"}
 _SCAN = {"linear_scan", "linear_scan_sm100", "conv1d", "conv_any"}
 KIND_KERNELS = {

@@ -61,6 +61,11 @@ __device__ __forceinline__ float xielu_fast(float z, float a, float b) {
   const float p = fmaxf(z, 0.f);
   return fmaf(a * p, p, fmaf(b, e, 0.5f * z));
 }
+// activation of a gate: 0 = silu, 1 = gelu (tanh form)
+__device__ __forceinline__ float gate_act(float v, int act) {
+  if (act == 0) return v / (1.f + __expf(-v));
+  return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+}
 __device__ __forceinline__ float warp_sum_f(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

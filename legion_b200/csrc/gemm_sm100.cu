@@ -145,11 +145,6 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       : "memory");
 }
 
-__device__ __forceinline__ float gate_act(float v, int act) {
-  if (act == 0) return v / (1.f + __expf(-v));
-  return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-}
-
 // UNARY: the output passes xIELU with its two WgemmArgs::numbers, or max(., 0)^2; UN_BIAS: gate and up get their
 // biases (DUAL). Variants of their own, as is the
 // lookahead of output rows for wide token tiles: decode-sized launches run the epilogue once, and code they skip still
@@ -986,6 +981,9 @@ int g_num_sms = 0;
 
 }  // namespace
 
+bool wgemm_pair_ok(const WgemmHost& h, const WgemmArgs& a, int sms);
+int wgemm_pair_launch(const WgemmHost& h, const WgemmArgs& a, int sms, cudaStream_t stream, const char** err);
+
 int wgemm_pick_bn(int n_tok_per_tile_hint, bool dual) {
   int bn = 32;
   while (bn < n_tok_per_tile_hint && bn < (dual ? 128 : 256)) bn *= 2;
@@ -1101,6 +1099,12 @@ int wgemm_launch(const WgemmHost& h, cudaStream_t stream) {
   if (total <= 0) return 0;
   int grid = int(total < g_num_sms ? total : g_num_sms);
 
+  if (wgemm_pair_ok(h, a, g_num_sms)) {
+    const char* err = nullptr;
+    if (wgemm_pair_launch(h, a, g_num_sms, stream, &err) == 0) return 0;
+    snprintf(g_gemm_err, sizeof(g_gemm_err), "wgemm: %s", err);
+    return 1;
+  }
 #define LB_CASE(BN_, DUAL_)                                                                     \
   if (bn == BN_ && h.dual == DUAL_) {                                                           \
     if (fp4) return launch<BN_, DUAL_, false, true>(tmW, tmX, tmS, a, grid, stream);            \

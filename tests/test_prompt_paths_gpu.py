@@ -66,3 +66,41 @@ def test_latent_prompt_per_head_form(lens, cached, monkeypatch):
     # two orders of bf16 roundings (keys and values against queries and attended latents), two layers
     assert (a - b).norm() < 0.01 * b.norm(), (a - b).norm() / b.norm()
     assert torch.equal(ka[0], kb[0]) and (ka[1] - kb[1]).norm() < 0.01 * kb[1].norm()
+
+
+# tiles of 256 tokens with a remainder, features that end inside a pair of SMs, a last K block that is not whole
+@pytest.mark.parametrize("T,N,K", [(1300, 4104, 584), (2304, 2560, 512), (1281, 4352, 1024)])
+def test_prompt_gemm_on_pairs(T, N, K):
+    x, w, res = _rnd(T, K), _rnd(N, K, scale=K ** -0.5, seed=1), _rnd(T, N, seed=2)
+    scale = torch.rand(T, generator=torch.Generator().manual_seed(3)).to(DEV)
+    want = x.double() @ w.double().t()
+    gate, up = want[:, :N // 2], want[:, N // 2:]
+    for out, exact in ((sm().linear(x, w), want), (sm().linear(x, w, residual=res), want + res.double()),
+                       (sm().linear(x, w, tok_scale=scale), want * scale.double()[:, None]),
+                       (sm().gate_up_act(x, w, N // 2), torch.nn.functional.silu(gate) * up)):
+        # fp32 sums of exact products of N(0, 1) values (about K^0.5 * 2^-24), fast exponential, one bf16 rounding
+        assert (out.double() - exact).abs().max() < 2.0 ** -8 * exact.abs().max()
+        assert (out.double() - exact).norm() < 2.0 ** -8 * exact.norm()
+    assert sm().Workspace.get(DEV).check() == 0
+
+
+# groups of 0, 1, 127, 128, 129 tokens and more over token tiles of 128, both expert products
+def test_grouped_gemm_on_pairs():
+    E, H, F = 24, 512, 640
+    counts = [0, 1, 127, 128, 129, 300] * 4
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])
+    ids = ids[torch.randperm(len(ids), generator=torch.Generator().manual_seed(0))].to(DEV)[:, None]
+    T = len(ids)
+    assert 64 * E < T <= 128 * E
+    x, gu, dn = _rnd(T, H), _rnd(E, 2 * F, H, scale=H ** -0.5, seed=1), _rnd(E, H, F, scale=F ** -0.5, seed=2)
+    wts = torch.rand(T, 1, generator=torch.Generator().manual_seed(4)).to(DEV)
+    out = sm().moe_experts(x, ids, wts, gu, dn, F).double()
+    assert sm().Workspace.get(DEV).check() == 0
+    want = torch.empty(T, H, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        t = (ids[:, 0] == e).nonzero()[:, 0]
+        a, b = (x[t].double() @ gu[e].double().t()).chunk(2, -1)
+        h = (torch.nn.functional.silu(a) * b).to(torch.bfloat16).double()
+        want[t] = (h @ dn[e].double().t()) * wts[t].double()
+    # three bf16 roundings: the activations (of values near a tie), the pair rows, the output
+    assert (out - want).norm() < 3 * 2.0 ** -9 * want.norm()
