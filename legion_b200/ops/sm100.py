@@ -7,6 +7,7 @@ The extension is required on a GPU: there is no silent fallback to eager PyTorch
 """
 from __future__ import annotations
 
+import functools
 import importlib
 import os
 import threading
@@ -129,6 +130,7 @@ for _kv in os.environ.get("LB_TUNE", "").split(","):
         TUNE[_kv.split("=")[0].strip()] = int(_kv.split("=")[1])
 
 
+SPLITK_FLOATS = 1 << 23
 _CANARY_ON = os.environ.get("LB_CANARY", "0") == "1"
 
 
@@ -144,7 +146,7 @@ class Workspace:
         self.device = device
         self.status = torch.zeros(4, dtype=torch.int32, device=device)
         self.counters = torch.zeros(1 << 16, dtype=torch.int32, device=device)
-        self.splitk = torch.empty(1 << 23, dtype=torch.float32, device=device)  # 32 MiB
+        self.splitk = torch.empty(SPLITK_FLOATS, dtype=torch.float32, device=device)  # 32 MiB
         self._attn: dict = {}
         self._cache: dict = {}
         self._guards: dict = {}
@@ -470,6 +472,34 @@ def pick_bn(n_tok: int, dual: bool) -> int:
     return bn
 
 
+@functools.lru_cache(maxsize=4096)
+def _pick_tile(T: int, n_feat: int, K: int, dual: bool):
+    """(token tile, K splits) of a bf16 GEMM with more than 32 tokens that does not fill the pairs of SMs
+    (``gemm_pair_sm100.cu``): the pair with the least modelled time, in cycles. A k block of 64 costs what its operands move
+    through shared memory in and out at 128 bytes per cycle, 32 columns of accumulators about 1400 cycles on their way out; a
+    split adds its partial sums. Short prompts otherwise ran as one wide token tile on a few SMs, or with their sums spread
+    over so many splits that adding those up took most of the time: 217 tokens, 2048 x 4096 weights, 34 us with 256-token
+    tiles in nine splits, 12 us with 64-token tiles in two."""
+    ft, nw, num_kb = (n_feat + 127) // 128, 2 if dual else 1, (K + 63) // 64
+    if T > 128 and ((T + 255) // 256) * ((nw * n_feat + 255) // 256) >= NUM_SMS // 2 and K >= 512:
+        return (128 if dual else 256), 1
+    best = None
+    for bn in (32, 64, 128) if dual else (32, 64, 128, 256):
+        if bn > 32 and bn // 2 >= T:
+            continue
+        tiles = ((T + bn - 1) // bn) * ft
+        for sk in (1, 2, 3, 4, 6, 8):
+            if sk > 1 and (num_kb < 4 * sk or tiles * sk > 2 * NUM_SMS or tiles * sk * bn * nw * 128 > SPLITK_FLOATS):
+                continue
+            waves, kbs = (tiles * sk + NUM_SMS - 1) // NUM_SMS, (num_kb + sk - 1) // sk
+            main = kbs * (16384 * nw + 128 * bn * nw + 16384 * nw + 128 * bn) // 128
+            out = bn // 32 * (1400 * nw if sk == 1 else nw * (700 + 500 * sk))
+            cost = 2500 + (waves * max(main, out) + min(main, out))
+            if best is None or cost < best[0]:
+                best = (cost, bn, sk)
+    return best[1], best[2]
+
+
 def _pick_split_k(n_tok_tiles: int, feat_tiles: int, K: int) -> int:
     """Split K when a skinny GEMM has too few tiles to keep the SMs streaming weights."""
     tiles = n_tok_tiles * feat_tiles
@@ -649,6 +679,8 @@ def linear(x, w, residual=None, out=None, out_dtype=torch.bfloat16, split_k: Opt
             raise ValueError("NVFP4 weights produce bf16 outputs")
         return linear_nv4(x if isinstance(x, Nv4Act) else nv4_quant_act(x), w, residual=residual, out=out)
     ws = Workspace.get(x.device)
+    if bn is None and split_k is None and T > 32 and not q:
+        bn, split_k = _pick_tile(T, N, K, False)
     bn = bn or pick_bn(T, False)
     n_tt = (T + bn - 1) // bn
     ft = (N + 127) // 128
@@ -683,6 +715,9 @@ def gate_up_act(x, w_gate_up, n_ff: int, out=None, bn=None, split_k: Optional[in
     if isinstance(w_gate_up, Nv4Weight):
         return gate_up_nv4(x if isinstance(x, Nv4Act) else nv4_quant_act(x), w_gate_up, n_ff, out=out)
     ws = Workspace.get(x.device)
+    q = isinstance(w_gate_up, QWeight)
+    if bn is None and split_k is None and T > 32 and not q:
+        bn, split_k = _pick_tile(T, n_ff, K, True)
     bn = bn or pick_bn(T, True)
     n_tt = (T + bn - 1) // bn
     ft = (n_ff + 127) // 128
@@ -691,7 +726,6 @@ def gate_up_act(x, w_gate_up, n_ff: int, out=None, bn=None, split_k: Optional[in
         need = C.wgemm_workspace_floats(bn, True, n_tt, ft, sk)
         if need > ws.splitk.numel() or n_tt * ft > ws.counters.numel():
             sk = 1
-    q = isinstance(w_gate_up, QWeight)
     C.wgemm(w_gate_up.codes if q else w_gate_up, x, out, None, None, None, n_ff, True, n_ff, bn, sk,
             ws.splitk if sk > 1 else None, ws.counters if sk > 1 else None, ws.status, None, None, None, None, 0, 0, T,
             [], None, w_gate_up.scales if q else None, w_gate_up.gscale if q else None, 0, 0, GATE_ACTS[act], bias=bias)

@@ -104,3 +104,14 @@ def test_grouped_gemm_on_pairs():
         want[t] = (h @ dn[e].double().t()) * wts[t].double()
     # three bf16 roundings: the activations (of values near a tie), the pair rows, the output
     assert (out - want).norm() < 3 * 2.0 ** -9 * want.norm()
+
+
+# token counts between decode steps and full tiles: every tile and split the dispatch takes
+@pytest.mark.parametrize("T", [33, 65, 217, 600])
+@pytest.mark.parametrize("N,K", [(1, 2048), (512, 2048), (2048, 4096), (12352, 2048), (576, 72)])
+def test_short_prompt_gemm(T, N, K):
+    x, w = _rnd(T, K), _rnd(N, K, scale=K ** -0.5, seed=1)
+    want = x.double() @ w.double().t()
+    for dt, eps in ((torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -18)):
+        assert (sm().linear(x, w, out_dtype=dt).double() - want).norm() < eps * want.norm()
+    assert sm().Workspace.get(DEV).check() == 0
