@@ -430,7 +430,7 @@ void bind_quant(pybind11::module_& m) {
                         const OptT& tok_scale, const OptT& out_rows, int64_t n_feat, bool dual, int64_t dual_offset,
                         int64_t act, int64_t bn, Tensor& status, const OptT& tile_group, const OptT& tile_tok0,
                         const OptT& tile_ntok, const OptT& meta, int64_t max_tiles, int64_t rows_per_group, int64_t n_tok,
-                        const OptT& tile_out0, const OptT& q_codes, const OptT& q_sf, const OptT& q_gscale) {
+                        const OptT& tile_out0, const OptT& q_codes, const OptT& q_sf, const OptT& q_gscale, bool few) {
     TORCH_CHECK(w.is_cuda() && w.dim() == 2 && x.dim() == 2 && w.element_size() == 1 && x.element_size() == 1 &&
                     w.stride(1) == 1 && x.stride(1) == 1 && w.size(1) == x.size(1),
                 "wgemm_nv4: w [rows, K / 2] and x [tokens, K / 2] are packed e2m1 bytes with the same K");
@@ -467,8 +467,13 @@ void bind_quant(pybind11::module_& m) {
     h.n_tiles_dev = optp<int>(meta); h.tile_out0 = optp<int>(tile_out0); h.n_tok_tiles_max = int(max_tiles);
     h.rows_per_group = int(rows_per_group); h.dual_offset = int(dual_offset);
     h.status = reinterpret_cast<int*>(status.data_ptr());
+    h.few = few;
     TORCH_CHECK(lb::wgemm_nv4_launch(h, cur_stream()) == 0, lb::wgemm_nv4_last_error());
-  });
+  }, py::arg("w"), py::arg("w_sf"), py::arg("w_gscale"), py::arg("x"), py::arg("x_sf"), py::arg("x_gscale"), py::arg("x_gs_stride"),
+        py::arg("out"), py::arg("residual"), py::arg("tok_scale"), py::arg("out_rows"), py::arg("n_feat"), py::arg("dual"),
+        py::arg("dual_offset"), py::arg("act"), py::arg("bn"), py::arg("status"), py::arg("tile_group"), py::arg("tile_tok0"),
+        py::arg("tile_ntok"), py::arg("meta"), py::arg("max_tiles"), py::arg("rows_per_group"), py::arg("n_tok"),
+        py::arg("tile_out0"), py::arg("q_codes"), py::arg("q_sf"), py::arg("q_gscale"), py::arg("few") = false);
   m.def("gguf_dequant", [](const Tensor& raw, int64_t ggml_type, Tensor& out) {
     TORCH_CHECK(raw.scalar_type() == at::kByte && raw.is_contiguous() && out.scalar_type() == at::kBFloat16 &&
                     out.is_contiguous(), "gguf_dequant: raw uint8 -> bf16");

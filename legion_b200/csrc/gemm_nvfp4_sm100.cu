@@ -82,7 +82,7 @@ struct Args {
   uint8_t* q_codes; long q_ld; uint8_t* q_sf; const float* q_gscale; int q_k4;
   int K, n_feat, feat_tiles, n_tok, k4;
   const int* tile_group; const int* tile_tok0; const int* tile_out0; const int* tile_ntok; const int* n_tiles_dev;
-  int n_tok_tiles_max, rows_per_group, dual_offset, act, vec_ok;
+  int n_tok_tiles_max, rows_per_group, dual_offset, act, vec_ok, few;
   int* status;
 };
 
@@ -128,6 +128,10 @@ __device__ __forceinline__ void umma_nvf4(uint32_t d_tmem, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
       : "memory");
+}
+// one accumulator column: thread i of the warp gets lane (base_lane + i)
+__device__ __forceinline__ void tmem_ld1(uint32_t taddr, uint32_t& r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
 }
 // Instruction descriptor: e2m1 x e2m1, UE4M3 scales, K-major operands, fp32 accumulate, K = 64.
 __host__ __device__ constexpr uint32_t nvf4_idesc(uint32_t M, uint32_t N) {
@@ -316,6 +320,51 @@ wgemm_nv4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     Work it, nx;
     const float q_gs = QOUT ? *a.q_gscale : 1.f;
     const float xs_all = (a.x_gscale && a.x_gs_stride == 0) ? __ldg(a.x_gscale) : 1.f;
+    // eight features of one output row: encoded (16 features = this thread and its neighbour: one scale byte, two words of codes)
+    // or weighted bf16 (+ residual)
+    auto put_row = [&](float (&v)[8], bool live, long orow, float sc, int feat8) {
+      if (QOUT) {
+        float amax = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        const uint32_t sb = e4m3_enc(amax / (6.f * q_gs));
+        const float sdec = e4m3_dec(sb) * q_gs;
+        const float inv = sdec > 0.f ? 1.f / sdec : 0.f;
+        if (live) {
+          *reinterpret_cast<uint32_t*>(a.q_codes + orow * a.q_ld + (feat8 >> 1)) = pack_e2m1x8(v, inv);
+          if ((etid & 1) == 0) a.q_sf[sf_atom_byte(orow, feat8 >> 4, a.q_k4)] = uint8_t(sb);
+        }
+      } else if (live && orow >= 0) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= sc;
+        if (a.vec_ok) {
+          if (a.residual) {
+            const uint4 rr = *reinterpret_cast<const uint4*>(a.residual + orow * a.ldr + feat8);
+            const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 f = __bfloat1622float2(r2[e]);
+              v[2 * e] += f.x;
+              v[2 * e + 1] += f.y;
+            }
+          }
+          uint4 o;
+          o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
+          o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+          *reinterpret_cast<uint4*>(a.out + orow * a.ldo + feat8) = o;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (feat8 + e < a.n_feat) {
+              float o = v[e];
+              if (a.residual) o += __bfloat162float(a.residual[orow * a.ldr + feat8 + e]);
+              a.out[orow * a.ldo + feat8 + e] = __float2bfloat16(o);
+            }
+          }
+        }
+      }
+    };
     bool have = decode_work<BN, FT>(a, blockIdx.x, n_tok_tiles, it);
     for (int w = blockIdx.x; have; w += gridDim.x, it = nx) {
       have = decode_work<BN, FT>(a, w + gridDim.x, n_tok_tiles, nx);
@@ -342,7 +391,22 @@ wgemm_nv4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         if (a.x_gscale && a.x_gs_stride != 0)
           xs_lane = (c + lane < it.ntok) ? __ldg(&a.x_gscale[long(it.tok0 + c + lane) * a.x_gs_stride]) : 1.f;
       };
-      prefetch_rows(eset * 32);
+      // Dense routing with 33 to 64 tokens: all of them are columns of every expert's tile, few chose the expert
+      // (out_rows >= 0), and only their columns are taken out of the accumulator. 64 users, 512 experts of 2048 x 512, 10 per
+      // token: a step of 8 layers takes 2.94 ms with this and two CTAs per SM, 3.13 ms as two halves with 32-token tiles that
+      // each read the weights. Tiles of 32 tokens gain nothing (16 users: gate and up 40 us with it, 37 without).
+      constexpr bool FEW = BN == 64 && !EPI2;
+      const bool few = FEW && a.few;
+      int my_row = -1;                                 // of column c + lane: output row, its weight
+      float my_sc = 1.f;
+      auto prefetch_few = [&](int c) {
+        const bool in = c + lane < it.ntok;
+        my_row = in ? a.out_rows[it.out0 + c + lane] : -1;
+        my_sc = (!QOUT && in && a.tok_scale) ? a.tok_scale[it.out0 + c + lane] : 1.f;
+        if (a.x_gscale && a.x_gs_stride != 0) xs_lane = in ? __ldg(&a.x_gscale[long(it.tok0 + c + lane) * a.x_gs_stride]) : 1.f;
+      };
+      if (few) prefetch_few(0);
+      else prefetch_rows(eset * 32);
       if (!__all_sync(0xffffffffu, mbar_wait(&tfull[acc], acc_ph, abort_flag))) {
         *abort_flag = 1;
         atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL);
@@ -360,7 +424,59 @@ wgemm_nv4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll 1
       for (int c = eset * 32; c < BN; c += 32 * C::NSETS) {
         if (c >= it.ntok) break;
-        if (c > eset * 32 || (f > 0 && BN > 32)) prefetch_rows(c);
+        if constexpr (FEW) {
+          if (few) {
+            if (c > 0) prefetch_few(c);
+            const unsigned cols = __ballot_sync(0xffffffffu, my_row >= 0);     // the same in all four warps
+            if (cols == 0) continue;
+            const int n = __popc(cols);
+            if (n <= 8) {
+              uint32_t g[8], u[8];
+              unsigned m = cols;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                if (i < n) {
+                  const int col = __ffs(m) - 1;
+                  m &= m - 1;
+                  tmem_ld1(t0 + c + col, g[i]);
+                  if (DUAL) tmem_ld1(t0 + BN + c + col, u[i]);
+                }
+              }
+              tmem_ld_wait();
+              m = cols;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                if (i < n) {
+                  const float xs = __shfl_sync(0xffffffffu, xs_lane, __ffs(m) - 1);
+                  m &= m - 1;
+                  float v = __uint_as_float(g[i]) * gs0 * xs;
+                  if (DUAL) {
+                    const float w = __uint_as_float(u[i]) * gs1 * xs;
+                    if (a.act == 0) v = (v / (1.f + __expf(-v))) * w;
+                    else v = 0.5f * v * (1.f + tanhf(0.7978845608f * (v + 0.044715f * v * v * v))) * w;
+                  }
+                  stage[i * BM + row] = v;
+                }
+              }
+              asm volatile("bar.sync 2, 128;" ::: "memory");
+              const int j = etid >> 4, f8 = (etid & 15) * 8, feat8 = it.feat0 + f8;
+              const bool live = j < n && feat8 < a.n_feat;
+              m = cols;
+              for (int i = 0; i < j; ++i) m &= m - 1;
+              const int col = m ? __ffs(m) - 1 : 0;                            // the row's column, of the j + 1-th set bit
+              const int mapped = __shfl_sync(0xffffffffu, my_row, col);
+              const float sc = __shfl_sync(0xffffffffu, my_sc, col);
+              const float4 v0 = *reinterpret_cast<const float4*>(&stage[j * BM + f8]);
+              const float4 v1 = *reinterpret_cast<const float4*>(&stage[j * BM + f8 + 4]);
+              float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+              put_row(v, live, QOUT ? long(it.out0 + c + col) : long(mapped), sc, feat8);
+              asm volatile("bar.sync 2, 128;" ::: "memory");
+              continue;
+            }
+            prefetch_rows(c);
+          }
+        }
+        if (!few && (c > eset * 32 || (f > 0 && BN > 32))) prefetch_rows(c);
         uint32_t r[32];
         float g[32];
         tmem_ld32(t0 + c, r);
@@ -394,53 +510,7 @@ wgemm_nv4_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           const float4 v0 = *reinterpret_cast<const float4*>(&stage[j * BM + f8]);
           const float4 v1 = *reinterpret_cast<const float4*>(&stage[j * BM + f8 + 4]);
           float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-          const int xrow = it.out0 + t;
-          if (QOUT) {
-            // 16 features = this thread and its neighbour: one scale byte, two words of codes
-            float amax = 0.f;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            const uint32_t sb = e4m3_enc(amax / (6.f * q_gs));
-            const float sdec = e4m3_dec(sb) * q_gs;
-            const float inv = sdec > 0.f ? 1.f / sdec : 0.f;
-            if (live) {
-              *reinterpret_cast<uint32_t*>(a.q_codes + long(xrow) * a.q_ld + (feat8 >> 1)) = pack_e2m1x8(v, inv);
-              if ((etid & 1) == 0) a.q_sf[sf_atom_byte(xrow, feat8 >> 4, a.q_k4)] = uint8_t(sb);
-            }
-          } else if (live) {
-            const long orow = orow_p[pass];
-            if (orow >= 0) {
-              const float sc = sc_p[pass];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[e] *= sc;
-              if (a.vec_ok) {
-                if (a.residual) {
-                  const uint4 rr = *reinterpret_cast<const uint4*>(a.residual + orow * a.ldr + feat8);
-                  const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rr);
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const float2 f = __bfloat1622float2(r2[e]);
-                    v[2 * e] += f.x;
-                    v[2 * e + 1] += f.y;
-                  }
-                }
-                uint4 o;
-                o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
-                o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
-                *reinterpret_cast<uint4*>(a.out + orow * a.ldo + feat8) = o;
-              } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  if (feat8 + e < a.n_feat) {
-                    float o = v[e];
-                    if (a.residual) o += __bfloat162float(a.residual[orow * a.ldr + feat8 + e]);
-                    a.out[orow * a.ldo + feat8 + e] = __float2bfloat16(o);
-                  }
-                }
-              }
-            }
-          }
+          put_row(v, live, QOUT ? long(it.out0 + t) : orow_p[pass], sc_p[pass], feat8);
         }
         if (eset == 0) asm volatile("bar.sync 2, 128;" ::: "memory");
         else asm volatile("bar.sync 3, 128;" ::: "memory");
@@ -502,13 +572,18 @@ int wgemm_nv4_launch(const Nv4Host& h, cudaStream_t stream) {
     snprintf(g_err, sizeof(g_err), "wgemm_nv4: groups (and the gate / up halves) must start on 128-row boundaries");
     return 1;
   }
-  if (qout && (h.n_feat % 16 != 0 || !h.q_sf || !h.q_gscale || (h.q_ld % 4) || h.out_rows || h.tok_scale || h.residual)) {
+  if (qout && (h.n_feat % 16 != 0 || !h.q_sf || !h.q_gscale || (h.q_ld % 4) || (h.out_rows && !h.few) || h.tok_scale ||
+               h.residual)) {
     snprintf(g_err, sizeof(g_err), "wgemm_nv4: a quantised output needs n_feat %% 16 == 0 and no row map / scale / residual");
     return 1;
   }
   if (!h.tile_group && h.bn == 32 && h.n_tok > 32) {
     snprintf(g_err, sizeof(g_err), "wgemm_nv4: 32-token tiles serve up to 32 tokens (their scale factors must start a "
                                    "128-row atom); use 64 or 128");
+    return 1;
+  }
+  if (h.few && (!h.out_rows || !h.tile_group || h.bn != 64)) {
+    snprintf(g_err, sizeof(g_err), "wgemm_nv4: sparse columns come with a tile list, a row map and token tiles of 64");
     return 1;
   }
   if (!qout && !h.out) {
@@ -538,7 +613,7 @@ int wgemm_nv4_launch(const Nv4Host& h, cudaStream_t stream) {
   a.tile_group = h.tile_group; a.tile_tok0 = h.tile_tok0; a.tile_out0 = h.tile_out0; a.tile_ntok = h.tile_ntok;
   a.n_tiles_dev = h.n_tiles_dev; a.n_tok_tiles_max = h.n_tok_tiles_max;
   a.rows_per_group = h.rows_per_group; a.dual_offset = h.dual_offset; a.act = h.act;
-  a.status = h.status;
+  a.status = h.status; a.few = h.few;
   a.vec_ok = (!qout && h.n_feat % 8 == 0 && h.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(h.out) & 15) == 0 &&
               (!h.residual || (h.ldr % 8 == 0 && (reinterpret_cast<uintptr_t>(h.residual) & 15) == 0))) ? 1 : 0;
   const int n_tok_tiles = h.tile_group ? h.n_tok_tiles_max : (h.n_tok + bn - 1) / bn;
@@ -549,20 +624,25 @@ int wgemm_nv4_launch(const Nv4Host& h, cudaStream_t stream) {
   // producer), not by bytes in flight: several CTAs per SM, each with a share of the shared memory and tensor
   // memory, fill the gaps. Measured on the 80B-A3B expert shapes at 16 tokens: gate/up 43 -> 34 us with two CTAs
   // per SM, down (K = 512: two stages per tile) 31 -> 22 -> 20 us with two / three.
-  const bool short_k = bn == 32 && !h.dual && !qout && num_kb <= 4 && a.feat_tiles >= 8;
-  const bool many_dual = bn == 32 && h.dual && qout && long(n_tok_tiles) * a.feat_tiles >= 2L * g_sms;
-  const int ncta = short_k ? 3 : (many_dual ? 2 : 1);
+  const bool small = bn == 32 || (bn == 64 && h.few);
+  const bool short_k = small && !h.dual && !qout && num_kb <= 4 && a.feat_tiles >= 8;
+  const bool many_dual = small && h.dual && qout && long(n_tok_tiles) * a.feat_tiles >= 2L * g_sms;
+  const int ncta = short_k && bn == 32 ? 3 : (short_k || many_dual ? 2 : 1);
   const int ft = 1;
   const long total = long(n_tok_tiles) * ((a.feat_tiles + ft - 1) / ft);
   if (total <= 0) return 0;
   const int slots = ncta * g_sms;
   const int grid = int(total < slots ? total : slots);
   // prompt-sized grouped steps with 64-token tiles: two epilogue warpgroups
-  const bool big = h.tile_group && bn == 64 && h.n_tok_tiles_max >= 256;
+  const bool big = h.tile_group && bn == 64 && h.n_tok_tiles_max >= 256 && !h.few;
   if (big && !h.dual && !qout) return launch<64, false, false, 1, 1, true>(tmW, tmX, a, grid, stream);
   if (big && h.dual && qout) return launch<64, true, true, 1, 1, true>(tmW, tmX, a, grid, stream);
-  if (short_k) return launch<32, false, false, 1, 3>(tmW, tmX, a, grid, stream);
-  if (many_dual) return launch<32, true, true, 1, 2>(tmW, tmX, a, grid, stream);
+  if (short_k)
+    return bn == 32 ? launch<32, false, false, 1, 3>(tmW, tmX, a, grid, stream)
+                    : launch<64, false, false, 1, 2>(tmW, tmX, a, grid, stream);
+  if (many_dual)
+    return bn == 32 ? launch<32, true, true, 1, 2>(tmW, tmX, a, grid, stream)
+                    : launch<64, true, true, 1, 2>(tmW, tmX, a, grid, stream);
 #define LB_NV4(BN_, DUAL_, FT_)                                                             \
   if (bn == BN_ && h.dual == DUAL_ && ft == FT_)                                            \
     return qout ? launch<BN_, DUAL_, true, FT_>(tmW, tmX, a, grid, stream)                  \

@@ -30,6 +30,9 @@ struct Nv4Host {
   const __nv_bfloat16* residual; long ldr;
   const float* tok_scale;
   const int* out_rows;
+  // dense routing of a decode step: a tile's columns are the tokens of the step, and out_rows also tells which of them take
+  // part (>= 0); the rows of the others may be left unwritten. With a quantised output out_rows is that and no row map.
+  bool few;
   // quantised output instead of bf16: the epilogue result re-encoded to NVFP4 for the next GEMM
   uint8_t* q_codes; long q_ld;                    // [rows, n_feat / 2] bytes, pitch q_ld bytes
   uint8_t* q_sf;                                  // its scale atoms (k4 from n_feat)

@@ -61,15 +61,12 @@ class DecodeGraphs:
         return off, o
 
     def _lanes(self, B: int) -> int:
-        """Concurrent lanes of a decode step: from 64 rows the batch runs as two independent halves on parallel
-        branches of the graph. Each half stays within the 32-token tiles that the decode-sized kernels are tuned
-        for (several CTAs per SM in the expert GEMMs, one dense-routing tile per expert), and the two chains fill
-        each other's gaps: 16.1 against 18.0 ms per step at 64 users of the 80B-A3B shape. Below that it loses: at
-        16 users two lanes of 8 took 8.7 ms against 6.8 ms, because every decode kernel occupies the whole machine
-        while it waits on its own dependent hand-overs, so the lanes alternate instead of overlapping. One lane also
+        """Concurrent lanes of a decode step: one. On request (``decode_lanes`` 2) the batch runs from 64 rows on as two
+        independent halves on parallel branches of the graph, which fill each other's gaps but read every weight twice. One
+        lane wins since its kernels have variants for 64 rows: 64 users, 8 layers of the 80B-A3B shape 2.94 against 3.20 ms, 4 of
+        the 30B-A3B 1.69 / 1.80, 4 dense layers of width 5120 1.43 / 1.56, 6 of latent attention 1.36 / 1.48. Never two
         for ranks that take part in collectives (their order must be the same on every rank), for offloaded experts, and
-        for models whose sublayers run on branches of their own (``Decoder._branch``): those fill the gaps without a second
-        pass over the weights (4.4 against 5.9 ms per step at 64 users of a 4B model)."""
+        for models whose sublayers run on branches of their own (``Decoder._branch``)."""
         eng = self.eng
         pc = eng.model.pctx
         if eng.mcfg.parallel_sublayers and ops.sm100.TUNE["parallel_branches"]:

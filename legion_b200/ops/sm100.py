@@ -124,7 +124,7 @@ def have_ext() -> bool:
 NUM_SMS = 148
 
 # tuning knobs (environment: LB_TUNE="decode_fixed_tiles=2,dense_route=1")
-TUNE = {"parallel_branches": 3, "decode_lanes": 2, "nv4_sorted": 1, "fp8_fused_quant": 1, "nv4_sorted_bn": 64, "gdn_chunk": 1, "decode_fixed_tiles": 2, "fused_plan": 1, "fused_router": 1, "dense_route": 1, "pdl": 1, "route_norm": 0, "mla_head_gemm": 1}
+TUNE = {"parallel_branches": 3, "decode_lanes": 1, "nv4_sorted": 1, "fp8_fused_quant": 1, "nv4_sorted_bn": 64, "gdn_chunk": 1, "decode_fixed_tiles": 2, "fused_plan": 1, "fused_router": 1, "dense_route": 1, "pdl": 1, "route_norm": 0, "mla_head_gemm": 1}
 for _kv in os.environ.get("LB_TUNE", "").split(","):
     if "=" in _kv:
         TUNE[_kv.split("=")[0].strip()] = int(_kv.split("=")[1])
@@ -1343,12 +1343,14 @@ def _moe_experts_nv4(x, ids, wts, w_gate_up: "Nv4Weight", w_down: "Nv4Weight", n
                  torch.zeros(C.nv4_sf_bytes(rows, n_ff), dtype=torch.uint8, device=x.device))
     hq_codes, hq_sf = dr.hq
     y_pairs = _dense_pairs(dr, P, T, k, H, x.device)
+    slots = min(dr.n_slots, P + int(routing.shared_slot))          # experts a step of P pairs can reach
+    few = dr.bn == 64
     C.wgemm_nv4(w_gate_up.view2d(), w_gate_up.sf, w_gate_up.gscale, xq.codes, xq.sf, xq.gscale, xq.stride, None, None,
-                None, None, n_ff, True, n_ff, 0, dr.bn, ws.status, dr.tile_group, dr.zeros, dr.tile_ntok, dr.meta,
-                dr.n_slots, 2 * n_ff, 0, dr.slot_base, hq_codes, hq_sf, h_scale)
+                None, dr.out_rows if few else None, n_ff, True, n_ff, 0, dr.bn, ws.status, dr.tile_group, dr.zeros, dr.tile_ntok, dr.meta,
+                slots, 2 * n_ff, 0, dr.slot_base, hq_codes, hq_sf, h_scale, few=few)
     C.wgemm_nv4(w_down.view2d(), w_down.sf, w_down.gscale, hq_codes, hq_sf, h_scale, 0, y_pairs, None, dr.tok_scale,
                 dr.out_rows, H, False, 0, 0, dr.bn, ws.status, dr.tile_group, dr.slot_base, dr.tile_ntok, dr.meta,
-                dr.n_slots, H, 0, None, None, None, None)
+                slots, H, 0, None, None, None, None, few=few)
     return _dense_combine(dr, routing, ids, e_lo, T, k, H, shared, shared_gate, residual, out, norm, x.device, defer)
 
 
