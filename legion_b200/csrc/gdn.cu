@@ -245,21 +245,25 @@ int gdn_recurrent_launch(const void* qkv, long ld, const float* g, const float* 
 
 // Decode step of a Gated DeltaNet layer in ONE launch: causal conv + SiLU of this token's q / k / v channels (with
 // the carried history), gates, the delta-rule update of the state, and the gated RMS norm of the output. One CTA
-// per (key head, sequence) serves the r = Hv / Hk value heads that share the key head (256 threads each), so the
+// per (key head, sequence) serves the r = Hv / Hk value heads that share the key head (NS x DV threads each), so the
 // q / k convolution, their L2 norms and the conv-history update are done once and nobody reads a history another
 // CTA is rewriting. Every sequence contributes exactly one token (row `seq` of proj).
+// Bound by the state, read and written once (2 x 2 MB per sequence for 32 heads of 128 x 128), as long as it stays in
+// registers: a thread holds DK / NS cells of one column. Two value heads take 1024 threads of 32 cells; 512 threads of 64
+// cells, compiled for blocks of up to 1024, had 64 registers and spilled: 64 / 16 / 1 sequences took 94 / 24 / 11 us, now
+// 66 / 17 / 7 (42 us is what the state of 64 takes at 6.46 TB/s).
 //   proj row = [q (Hk*DK) | k (Hk*DK) | v (Hv*DV) | z (Hv*DV) | b (Hv) | a (Hv)]  (the fused input projection)
 // Intermediate values are rounded to bf16 where the separate kernels store them as bf16 (conv outputs, the
 // recurrence output), so a decode step gives the same numbers as the multi-kernel path used for verify rows.
-template <int DK, int DV, int KC>
-__global__ void __launch_bounds__(1024) gdn_decode_fused_kernel(
+template <int DK, int DV, int KC, int NS, int THREADS>
+__global__ void __launch_bounds__(THREADS) gdn_decode_fused_kernel(
     const __nv_bfloat16* __restrict__ proj, long ld, const float* __restrict__ conv_w, float* __restrict__ conv_state,
     const float* __restrict__ A, const float* __restrict__ dt_bias, const float* __restrict__ norm_w, float eps,
     int act, float* __restrict__ state, const int* __restrict__ slots, int Hk, int Hv, int tiled_heads, float scale,
     float l2_eps, __nv_bfloat16* __restrict__ out) {
   static_assert(DK == DV, "thread layout assumes square heads");
-  constexpr int HALF = DK / 2;
-  constexpr int GT = 2 * DV;                     // threads per value head
+  constexpr int CELLS = DK / NS;
+  constexpr int GT = NS * DV;                    // threads per value head
   constexpr int MAXR = 4;
   griddep_wait();
   griddep_launch();
@@ -267,17 +271,17 @@ __global__ void __launch_bounds__(1024) gdn_decode_fused_kernel(
   const int r = Hv / Hk;
   const int j = threadIdx.x / GT, tid = threadIdx.x % GT;
   const int h = tiled_heads ? kh + j * Hk : kh * r + j;
-  const int c = tid % DV, half = tid / DV;
+  const int c = tid % DV, part_i = tid / DV;
   const int C = 2 * Hk * DK + Hv * DV;
   const int slot = slots[seq];
   const __nv_bfloat16* row = proj + long(seq) * ld;
-  __shared__ float q_s[DK], k_s[DK], v_s[MAXR][DV], part[MAXR][2][DV], red[2 * DK / 32], red2[MAXR][DV / 32];
+  __shared__ float q_s[DK], k_s[DK], v_s[MAXR][DV], part[MAXR][NS][DV], red[2 * DK / 32], red2[MAXR][DV / 32];
   __shared__ float qn_s, kn_s;
-  // state of this thread's half column: the loads are in flight while the convolution runs
-  float S[HALF];
-  float* sp = state + ((long(slot) * Hv + h) * DK + half * HALF) * DV + c;
+  // this thread's part of a state column: the loads are in flight while the convolution runs
+  float S[CELLS];
+  float* sp = state + ((long(slot) * Hv + h) * DK + part_i * CELLS) * DV + c;
 #pragma unroll
-  for (int i = 0; i < HALF; ++i) S[i] = sp[long(i) * DV];
+  for (int i = 0; i < CELLS; ++i) S[i] = sp[long(i) * DV];
 
   auto conv = [&](int ch) -> float {
     float wv[KC], hh[KC - 1];
@@ -296,18 +300,18 @@ __global__ void __launch_bounds__(1024) gdn_decode_fused_kernel(
     return __bfloat162float(__float2bfloat16(acc / (1.f + __expf(-acc))));
   };
   float qq = 0.f, kk = 0.f;
-  if (j == 0) {
+  if (j == 0 && part_i < 2) {
     // threads 0 .. DK-1: q channel, DK .. 2 DK-1: k channel of this key head
-    const float v = conv((half == 0 ? 0 : Hk * DK) + kh * DK + c);
-    if (half == 0) { q_s[c] = v; qq = v * v; } else { k_s[c] = v; kk = v * v; }
+    const float v = conv((part_i == 0 ? 0 : Hk * DK) + kh * DK + c);
+    if (part_i == 0) { q_s[c] = v; qq = v * v; } else { k_s[c] = v; kk = v * v; }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       qq += __shfl_xor_sync(0xffffffffu, qq, o);
       kk += __shfl_xor_sync(0xffffffffu, kk, o);
     }
-    if ((tid & 31) == 0) red[tid >> 5] = half == 0 ? qq : kk;
+    if ((tid & 31) == 0) red[tid >> 5] = part_i == 0 ? qq : kk;
   }
-  if (half == 0) v_s[j][c] = conv(2 * Hk * DK + h * DV + c);
+  if (part_i == (NS > 2 ? 2 : 0)) v_s[j][c] = conv(2 * Hk * DK + h * DV + c);
   __syncthreads();
   if (threadIdx.x == 0) {
     float a = 0.f, b = 0.f;
@@ -324,32 +328,37 @@ __global__ void __launch_bounds__(1024) gdn_decode_fused_kernel(
   const float qn = qn_s, kn = kn_s;
   float kv = 0.f;
 #pragma unroll
-  for (int i = 0; i < HALF; ++i) kv += S[i] * k_s[half * HALF + i];
-  part[j][half][c] = kv * kn;
+  for (int i = 0; i < CELLS; ++i) kv += S[i] * k_s[part_i * CELLS + i];
+  part[j][part_i][c] = kv * kn;
   __syncthreads();
-  const float delta = (v_s[j][c] - gt * (part[j][0][c] + part[j][1][c])) * bt;
+  auto sum = [&]() {
+    float v = part[j][0][c] + part[j][1][c];
+    if constexpr (NS == 4) v += part[j][2][c] + part[j][3][c];
+    return v;
+  };
+  const float delta = (v_s[j][c] - gt * sum()) * bt;
   __syncthreads();
   float o = 0.f;
 #pragma unroll
-  for (int i = 0; i < HALF; ++i) {
-    S[i] = gt * S[i] + k_s[half * HALF + i] * kn * delta;
-    o += S[i] * q_s[half * HALF + i];
+  for (int i = 0; i < CELLS; ++i) {
+    S[i] = gt * S[i] + k_s[part_i * CELLS + i] * kn * delta;
+    o += S[i] * q_s[part_i * CELLS + i];
   }
-  part[j][half][c] = o * qn;
+  part[j][part_i][c] = o * qn;
 #pragma unroll
-  for (int i = 0; i < HALF; ++i) sp[long(i) * DV] = S[i];
+  for (int i = 0; i < CELLS; ++i) sp[long(i) * DV] = S[i];
   __syncthreads();
   // gated RMS norm over the head's DV outputs
   float ov = 0.f, ss = 0.f;
-  if (half == 0) {
-    ov = __bfloat162float(__float2bfloat16(part[j][0][c] + part[j][1][c]));
+  if (part_i == 0) {
+    ov = __bfloat162float(__float2bfloat16(sum()));
     ss = ov * ov;
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
     if ((c & 31) == 0) red2[j][c >> 5] = ss;
   }
   __syncthreads();
-  if (half == 0) {
+  if (part_i == 0) {
     float tot = 0.f;
 #pragma unroll
     for (int i = 0; i < DV / 32; ++i) tot += red2[j][i];
@@ -368,14 +377,15 @@ int gdn_decode_fused_launch(const void* proj, long ld, const float* conv_w, floa
   if (Hk <= 0 || Hv % Hk || Hv / Hk > 4 || KC != 4) return 1;
   const int r = Hv / Hk;
   dim3 grid(Hk, n_seqs);
-#define LB_GF(D_)                                                                                                   \
-  if (DK == D_ && DV == D_) {                                                                                       \
-    launch_pdl(gdn_decode_fused_kernel<D_, D_, 4>, grid, dim3(2 * D_ * r), 0, s,                                    \
+  // threads per column of a head: four where a block of all the key head's value heads has room for them, else two
+#define LB_GF(D_, R_, NS_, THREADS_)                                                                                \
+  if (DK == D_ && DV == D_ && r <= R_) {                                                                            \
+    launch_pdl(gdn_decode_fused_kernel<D_, D_, 4, NS_, THREADS_>, grid, dim3(NS_ * D_ * r), 0, s,                   \
                static_cast<const __nv_bfloat16*>(proj), ld, conv_w, conv_state, A, dt_bias, norm_w, eps, act, state, \
                slots, Hk, Hv, tiled_heads, scale, l2_eps, static_cast<__nv_bfloat16*>(out));                        \
     return cudaGetLastError() != cudaSuccess;                                                                       \
   }
-  LB_GF(128) LB_GF(64)
+  LB_GF(128, 1, 4, 512) LB_GF(128, 2, 4, 1024) LB_GF(128, 4, 2, 1024) LB_GF(64, 2, 4, 512) LB_GF(64, 4, 4, 1024)
 #undef LB_GF
   return 1;
 }
