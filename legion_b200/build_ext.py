@@ -61,11 +61,11 @@ def _run(cmd: list[str]) -> str:
 # loaded with lazy binding, so the absent ones do not matter until something calls them.
 CORE_TARGET = ROOT / "_C_core.so"
 CORE = {"gemm_sm100", "gemm_pair_sm100", "sgemm", "elementwise", "sampling", "spec", "tmap", "logits", "bindings", "bindings_layers"}
-_ATTN = {"attn_prefill_sm100", "attn_decode_sm100", "attn_decode", "attn_general"}
+_ATTN = {"attn_prefill_sm100", "attn_pair_sm100", "attn_decode_sm100", "attn_decode", "attn_general"}
 _SCAN = {"linear_scan", "linear_scan_sm100", "conv1d", "conv_any"}
 KIND_KERNELS = {
     "attn": _ATTN, "lightning": _SCAN, "ssd": _SCAN, "hgrn2": {"forget_scan", "forget_scan_sm100"},
-    "latent": {"attn_mla_sm100", "latent_attn", "attn_prefill_sm100", "attn_decode", "attn_general"},
+    "latent": {"attn_mla_sm100", "latent_attn", "attn_prefill_sm100", "attn_pair_sm100", "attn_decode", "attn_general"},
     "rglru": {"diag_scan", "conv1d", "conv_any"},
     "channel_delta": {"channel_delta", "channel_delta_mma"},
 }

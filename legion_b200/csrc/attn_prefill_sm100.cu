@@ -522,6 +522,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
 }
 
+int pair_attn_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const int* cu_q, const int* ctx_lens,
+                     const int* block_table, int table_width, int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk,
+                     int dv, float scale_log2, void* out, int* status, cudaStream_t s);
+
 namespace {
 thread_local char g_attn_err[256];
 
@@ -594,6 +598,13 @@ int prefill_attn_launch(const void* q, long T, const void* k_cache, const void* 
     a.scale_log2 = 2.f * 1.4426950408889634f * softcap;
   }
   a.out = static_cast<__nv_bfloat16*>(out); a.dk = dk; a.dv = dv; a.status = status;
+  // plain causal prompts of more than one tile of rows: pairs of SMs share keys and values (attn_pair_sm100.cu)
+  if (!x.on && !cap && window == 0 && causal && max_q_len > 128) {
+    const int rc = pair_attn_launch(tq, tk, tv, cu_q, ctx_lens, block_table, table_width, page, n_seqs, max_q_len, Hq, Hkv, dk, dv,
+                                    a.scale_log2, out, status, s);
+    if (rc > 0) snprintf(g_attn_err, sizeof(g_attn_err), "prefill attention: launch on pairs: %s", cudaGetErrorString(cudaGetLastError()));
+    if (rc >= 0) return rc;
+  }
   dim3 grid((max_q_len + 127) / 128, Hq, n_seqs);
 #define LB_DIM(K_, V_, B_)                                                                   \
   if (DK == K_ && DV == V_)                                                                  \

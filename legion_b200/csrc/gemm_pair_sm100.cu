@@ -156,7 +156,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_EMPTY | SITE_GEMM);
           break;
         }
-        fence_cluster();
         tc_fence_after();
         const uint32_t d0 = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {

@@ -115,3 +115,29 @@ def test_short_prompt_gemm(T, N, K):
     for dt, eps in ((torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -18)):
         assert (sm().linear(x, w, out_dtype=dt).double() - want).norm() < eps * want.norm()
     assert sm().Workspace.get(DEV).check() == 0
+
+
+# pairs of 256 query rows: one row more than a tile, an empty second tile, full pairs, short sequences beside long ones, cached
+# tokens in front; blocks of 128 keys with a remainder; head sizes between and at the kernel's, pages of a part of its tiles
+@pytest.mark.parametrize("q_lens,cached,page", [([129], 0, 64), ([256, 1, 130], 70, 16), ([257, 511], 128, 32), ([700, 128], 333, 64)])
+@pytest.mark.parametrize("Hq,Hkv,dk,dv", [(4, 2, 128, 128), (2, 2, 192, 128), (8, 1, 256, 256), (2, 1, 136, 72), (2, 1, 232, 208)])
+def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
+    n, T = len(q_lens), sum(q_lens)
+    ctx = [q + cached for q in q_lens]
+    width = -(-max(ctx) // page)
+    k, v = _rnd(n * width, page, Hkv, dk, seed=1), _rnd(n * width, page, Hkv, dv, seed=2)
+    q = _rnd(T, Hq, dk, scale=2.0, seed=3)
+    bt = torch.randperm(n * width, generator=torch.Generator().manual_seed(0)).int().view(n, width).to(DEV)
+    cu = torch.tensor([sum(q_lens[:i]) for i in range(n + 1)], dtype=torch.int32, device=DEV)
+    out = sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5)
+    assert sm().Workspace.get(DEV).check() == 0
+    for i in range(n):
+        kk = k[bt[i].long()].reshape(-1, Hkv, dk)[:ctx[i]].double().repeat_interleave(Hq // Hkv, 1)
+        vv = v[bt[i].long()].reshape(-1, Hkv, dv)[:ctx[i]].double().repeat_interleave(Hq // Hkv, 1)
+        a, b = sum(q_lens[:i]), sum(q_lens[:i + 1])
+        s = torch.einsum("qhd,khd->hqk", q[a:b].double(), kk) * dk ** -0.5
+        later = torch.arange(ctx[i], device=DEV)[None] > torch.arange(cached, ctx[i], device=DEV)[:, None]
+        want = torch.einsum("hqk,khd->qhd", s.masked_fill(later, float("-inf")).softmax(-1), vv)
+        # bf16 probabilities and output, 2^-9 each; single rows up to 2^-6 of the largest value
+        assert (out[a:b].double() - want).norm() < 2.0 ** -8 * want.norm()
+        assert (out[a:b].double() - want).abs().max() < 2.0 ** -6 * want.abs().max()
