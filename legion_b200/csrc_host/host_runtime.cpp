@@ -3,6 +3,7 @@
 //   RadixCache  compressed radix tree over whole blocks of token ids (match + lock, insert, LRU eviction)
 //   table_slots flat KV cell index of every position of a step (block table -> slots)
 //   pack_decode the packed int32 input record of a CUDA-graph decode step
+//   pack_step   the input record of any other step
 // Semantics are those of the Python classes in legion_b200/kv (which remain as the fallback and the executable
 // specification: tests/test_kv.py runs both). Counterparts in the reference: src/kv/blocks.rs, src/kv/radix.rs.
 #include <pybind11/numpy.h>
@@ -321,6 +322,55 @@ static void pack_decode(py::array_t<int32_t, py::array::c_style> buf, int B, int
   }
 }
 
+// Per-token and per-sequence inputs of a step, int32 words at the given offsets of the record: slots and logit rows (int64, two
+// words each), token ids, positions, cu_q, ctx_lens, state slots, block table [sequences, W]. `first` are the sequences' first
+// positions; `rope` their rotary positions where those are not the token positions (else None). The lists are read in place:
+// an 8192-token step took 1 ms when every one of its tensors was made from a Python list and copied by itself.
+static void pack_step(py::array_t<int32_t, py::array::c_style> buf, const std::vector<long>& off, int W, int block_size,
+                      const py::list& tokens, const std::vector<long>& first, const py::list& rope, const py::list& tables,
+                      const std::vector<int>& state_slots, const std::vector<long>& logit_rows) {
+  const size_t n = first.size();
+  if (off.size() != 8 || tokens.size() != n || rope.size() != n || tables.size() != n || state_slots.size() != n)
+    throw std::invalid_argument("pack_step: inconsistent row counts");
+  long T = 0;
+  for (size_t i = 0; i < n; ++i) T += long(py::list(tokens[i]).size());
+  const long words[8] = {2 * T, 2 * long(logit_rows.size()), T, T, long(n) + 1, long(n), long(n), long(n) * W};
+  for (int i = 0; i < 8; ++i)
+    if (off[size_t(i)] < 0 || off[size_t(i)] + words[i] > long(buf.size()) || (i < 2 && off[size_t(i)] % 2))
+      throw std::invalid_argument("pack_step: offsets");
+  int32_t* w = buf.mutable_data();
+  auto* slots = reinterpret_cast<int64_t*>(w + off[0]);
+  auto* lrows = reinterpret_cast<int64_t*>(w + off[1]);
+  int32_t *tok = w + off[2], *pos = w + off[3], *cu = w + off[4], *ctx = w + off[5], *st = w + off[6], *bt = w + off[7];
+  auto number = [](PyObject* list, Py_ssize_t i) {
+    const long v = PyLong_AsLong(PyList_GET_ITEM(list, i));
+    if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
+    return v;
+  };
+  std::copy(logit_rows.begin(), logit_rows.end(), lrows);
+  std::memset(bt, 0, sizeof(int32_t) * n * size_t(W));
+  long t = 0;
+  cu[0] = 0;
+  for (size_t i = 0; i < n; ++i) {
+    const py::list ids(tokens[i]), table(tables[i]);
+    const long m = long(ids.size()), blocks = (first[i] + m + block_size - 1) / block_size;
+    if (blocks > long(table.size()) || blocks > W) throw std::out_of_range("position beyond the block table");
+    for (long j = 0; j < blocks; ++j) bt[i * size_t(W) + size_t(j)] = int32_t(number(table.ptr(), j));
+    const bool own = !rope[i].is_none();
+    const py::list turned = own ? py::list(rope[i]) : py::list();
+    if (own && long(turned.size()) != m) throw std::invalid_argument("pack_step: rotary positions");
+    for (long j = 0; j < m; ++j, ++t) {
+      const long p = first[i] + j;
+      tok[t] = int32_t(number(ids.ptr(), j));
+      pos[t] = own ? int32_t(number(turned.ptr(), j)) : int32_t(p);
+      slots[t] = int64_t(bt[i * size_t(W) + size_t(p / block_size)]) * block_size + p % block_size;
+    }
+    cu[i + 1] = int32_t(t);
+    ctx[i] = int32_t(first[i] + m);
+    st[i] = state_slots[i];
+  }
+}
+
 // Byte-pair merges of one pre-tokenised word (byte-to-unicode mapped text): lowest-rank adjacent pair first, until no
 // pair has a rank; pieces that are not in the vocabulary fall back to their single symbols.
 // Same procedure as BpeTokenizer._bpe in legion_b200/loaders/tokenizer.py (reference: src/tokenizer/bpe.rs).
@@ -465,4 +515,5 @@ PYBIND11_MODULE(_host, m) {
       });
   m.def("table_slots", &table_slots);
   m.def("pack_decode", &pack_decode);
+  m.def("pack_step", &pack_step);
 }

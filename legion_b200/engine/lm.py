@@ -25,6 +25,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 import torch
 
 from ..config import ModelConfig
+from ..kv import blocks as kv_blocks
 from ..kv.blocks import BlockPool, BlockTable, OutOfBlocks
 from ..kv.radix import RadixCache
 from ..kv.saved_states import SavedStates
@@ -1021,50 +1022,61 @@ class LmEngine(Engine):
         from ..ops import sm100
         return sm100.mla_supported(model.n_head_l, self.mcfg.kv_lora, self.mcfg.qk_rope_dim, c.block_size)
 
-    def build_batch(self, rows: Sequence[Tuple[Seq, int, int]], write_state: bool = True) -> StepBatch:
-        dev = self.device
-        tok: List[int] = []
-        pos: List[int] = []
-        slots: List[int] = []
+    def _step_inputs(self, items, logit_rows: List[int], write_state: bool = True) -> StepBatch:
+        """items = [(seq, first position, its tokens)]: the tensors of a step as parts of one record, filled by the native host
+        runtime where it is built and brought to the device by one copy."""
+        pool, n = self.pool, len(items)
+        first = [p0 for _, p0, _ in items]
+        rope = [None if s.media is None else [s.rope_pos(p) for p in range(p0, p0 + len(t))] for s, p0, t in items]
         cu = [0]
-        ctx: List[int] = []
-        logit_rows: List[int] = []
-        width = 1
+        for _, _, t in items:
+            cu.append(cu[-1] + len(t))
+        T, ctx = cu[-1], [p0 + len(t) for _, p0, t in items]
+        width = max([1] + [pool.blocks_for(c) for c in ctx])
+        words = (2 * T, 2 * len(logit_rows), T, T, n + 1, n, n, n * width)
+        off = [0]
+        for m in words:
+            off.append(off[-1] + -(-m // 64) * 64)              # parts start on 256 bytes
+        cuda = self.device.type == "cuda"
+        host = torch.empty(off[-1], dtype=torch.int32, pin_memory=cuda)
+        if kv_blocks.NATIVE is not None:
+            kv_blocks.NATIVE.pack_step(host.numpy(), off[:-1], width, pool.block_size, [list(t) for _, _, t in items], first, rope,
+                                       [s.table.blocks for s, _, _ in items], [s.slot for s, _, _ in items], list(logit_rows))
+        else:
+            slots = [c for s, p0, t in items for c in s.table.slots(pool, p0, len(t))]
+            table = torch.zeros(n, width, dtype=torch.int32)
+            for i, (s, _, _) in enumerate(items):
+                nb = pool.blocks_for(ctx[i])
+                table[i, :nb] = torch.tensor(s.table.blocks[:nb], dtype=torch.int32)
+            pos = [p for r, p0, (_, _, t) in zip(rope, first, items) for p in (range(p0, p0 + len(t)) if r is None else r)]
+            i64 = [torch.tensor(v, dtype=torch.int64).view(torch.int32) for v in (slots, list(logit_rows))]
+            i32 = [torch.tensor(v, dtype=torch.int32) for v in ([x for _, _, t in items for x in t], pos, cu, ctx,
+                                                                [s.slot for s, _, _ in items])]
+            for o, part in zip(off, (*i64, *i32, table.view(-1))):
+                host[o:o + part.numel()] = part
+        rec = host.to(self.device, non_blocking=True) if cuda else host
+        slots, lrows, tok, pos, cu_t, ctx_t, states, table = (rec[o:o + m] for o, m in zip(off, words))
+        return StepBatch(token_ids=tok, positions=pos, cu_q=cu_t, ctx_lens=ctx_t, block_table=table.view(n, width),
+                         slots=slots.view(torch.int64), state_slots=states, logit_rows=lrows.view(torch.int64),
+                         max_q_len=max(len(t) for _, _, t in items), max_ctx=max(ctx), write_state=write_state, cu_q_host=cu,
+                         ctx_host=ctx)
+
+    def build_batch(self, rows: Sequence[Tuple[Seq, int, int]], write_state: bool = True) -> StepBatch:
+        items, logit_rows, base = [], [], 0
         for s, p0, n in rows:
             if s.phase == "decode":
-                toks = [s.tokens[-1]] + s.drafts[:n - 1]
-            else:
-                toks = s.tokens[p0:p0 + n]
-            tok.extend(toks)
-            if s.media is None:
-                pos.extend(range(p0, p0 + n))
-            else:
-                pos.extend(s.rope_pos(p) for p in range(p0, p0 + n))
-            slots.extend(s.table.slots(self.pool, p0, n))
-            base = cu[-1]
-            cu.append(base + n)
-            ctx.append(p0 + n)
-            width = max(width, self.pool.blocks_for(p0 + n))
-            if s.phase == "decode":
+                items.append((s, p0, [s.tokens[-1]] + s.drafts[:n - 1]))
                 logit_rows.extend(range(base, base + n))
-            elif p0 + n == s.n_prompt:
-                logit_rows.append(base + n - 1)
-        bt = torch.zeros(len(rows), width, dtype=torch.int32)
-        for i, (s, p0, n) in enumerate(rows):
-            nb = self.pool.blocks_for(p0 + n)
-            bt[i, :nb] = torch.tensor(s.table.blocks[:nb], dtype=torch.int32)
-        i32 = dict(dtype=torch.int32, device=dev)
-        b = StepBatch(
-            token_ids=torch.tensor(tok, **i32), positions=torch.tensor(pos, **i32), cu_q=torch.tensor(cu, **i32),
-            ctx_lens=torch.tensor(ctx, **i32), block_table=bt.to(dev),
-            slots=torch.tensor(slots, dtype=torch.int64, device=dev),
-            state_slots=torch.tensor([s.slot for s, _, _ in rows], **i32),
-            logit_rows=torch.tensor(logit_rows, dtype=torch.int64, device=dev),
-            max_q_len=max(n for _, _, n in rows), max_ctx=max(ctx), write_state=write_state, cu_q_host=cu, ctx_host=ctx)
+            else:
+                items.append((s, p0, s.tokens[p0:p0 + n]))
+                if p0 + n == s.n_prompt:
+                    logit_rows.append(base + n - 1)
+            base += n
+        b = self._step_inputs(items, logit_rows, write_state)
         if any(s.media is not None and s.phase != "decode" for s, _, _ in rows):
-            self._media_inputs(b, rows, tok)
+            self._media_inputs(b, rows, [t for _, _, toks in items for t in toks])
         if self.ring_len:
-            self._ring_inputs(b, [(s, p0, n) for s, p0, n in rows], width)
+            self._ring_inputs(b, [(s, p0, n) for s, p0, n in rows], b.block_table.shape[1])
         return b
 
     def _ring_inputs(self, b: StepBatch, rows, width: int) -> None:
@@ -1085,31 +1097,14 @@ class LmEngine(Engine):
         """items = [(seq, first position, token list)]: a batch over the sequences' own block tables with
         explicit tokens (drafters fill their KV and chain drafts with it). Logits: last row of each item, or the
         given rows of the batch."""
-        dev = self.device
-        tok, pos, slots, cu, ctx, lrows = [], [], [], [0], [], []
-        width = 1
-        for s, p0, toks in items:
-            n = len(toks)
-            tok.extend(toks)
-            pos.extend(range(p0, p0 + n) if s.media is None else (s.rope_pos(p) for p in range(p0, p0 + n)))
-            slots.extend(s.table.slots(self.pool, p0, n))
-            cu.append(cu[-1] + n)
-            ctx.append(p0 + n)
-            width = max(width, self.pool.blocks_for(p0 + n))
-            lrows.extend(range(cu[-2], cu[-1]) if all_logits else [cu[-1] - 1])
-        bt = torch.zeros(len(items), width, dtype=torch.int32)
-        for i, (s, p0, toks) in enumerate(items):
-            nb = self.pool.blocks_for(p0 + len(toks))
-            bt[i, :nb] = torch.tensor(s.table.blocks[:nb], dtype=torch.int32)
-        i32 = dict(dtype=torch.int32, device=dev)
-        b = StepBatch(token_ids=torch.tensor(tok, **i32), positions=torch.tensor(pos, **i32),
-                      cu_q=torch.tensor(cu, **i32), ctx_lens=torch.tensor(ctx, **i32), block_table=bt.to(dev),
-                      slots=torch.tensor(slots, dtype=torch.int64, device=dev),
-                      state_slots=torch.tensor([s.slot for s, _, _ in items], **i32),
-                      logit_rows=torch.tensor(lrows if logit_rows is None else logit_rows, dtype=torch.int64, device=dev),
-                      max_q_len=max(len(t) for _, _, t in items), max_ctx=max(ctx), cu_q_host=cu, ctx_host=ctx)
+        if logit_rows is None:
+            logit_rows, base = [], 0
+            for _, _, toks in items:
+                logit_rows.extend(range(base, base + len(toks)) if all_logits else [base + len(toks) - 1])
+                base += len(toks)
+        b = self._step_inputs(items, logit_rows)
         if self.ring_len:
-            self._ring_inputs(b, [(s, p0, len(toks)) for s, p0, toks in items], width)
+            self._ring_inputs(b, [(s, p0, len(toks)) for s, p0, toks in items], b.block_table.shape[1])
         return b
 
     # ------------------------------------------------------------------ steps planned by the caller

@@ -58,6 +58,7 @@ class StepBatch:
     cu_q_host: Optional[List[int]] = None
     ctx_host: Optional[List[int]] = None         # ctx_lens on the host
     latent_parts: Optional[list] = None          # ops.sm100.latent_parts of this step
+    gdn_plan: Optional[tuple] = None             # ops.sm100.gdn_chunk_plan of this step
     decode_splits: Optional[int] = None
     replay: Optional[dict] = None                # verify steps: per-layer recurrent inputs kept for commit
     rope_table: Optional[torch.Tensor] = None    # [T, rot] per-token cos | sin rows (multi-section rotary positions of
@@ -529,7 +530,7 @@ class Decoder:
         if b.replay is not None:
             b.replay[il] = (mixed, g, beta)
         o = ops.gdn_recurrent(conv, g, beta, st.ssm[il], b.cu_q, b.state_slots, nk, nv, dk, dv, cfg.gdn_tiled_heads,
-                              dk ** -0.5, 1e-6, write_state=b.write_state, cu_host=b.cu_q_host)
+                              dk ** -0.5, 1e-6, write_state=b.write_state, cu_host=b.cu_q_host, step=b)
         n = ops.gated_rmsnorm(o, z, w[f"{p}.gdn.norm"], cfg.rms_eps, cfg.gdn_gate_act)
         return self.pctx.defer_linear(n.reshape(n.shape[0], -1), w[f"{p}.gdn.out"], lazy=True)
 

@@ -419,10 +419,10 @@ def gdn_gates(a, b, A, dt_bias):
 
 
 def gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps=1e-6,
-                  write_state=True, cu_host=None):
+                  write_state=True, cu_host=None, step=None):
     if _cuda(qkv):
         return _sm.gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps,
-                                 write_state, cu_host=cu_host)
+                                 write_state, cu_host=cu_host, step=step)
     return _ref.gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps,
                               write_state)
 

@@ -1724,7 +1724,8 @@ def gdn_gates(a, b, A, dt_bias):
 
 
 def gdn_chunk_plan(cu_host, device):
-    """Host-side tables of the chunked scan for one step: 128-token blocks and per-sequence chunk ranges."""
+    """Tables of the chunked scan for one step, 128-token blocks and per-sequence chunk ranges: parts of one tensor, and one
+    copy to the device, that the layers of the step share (six copies in every layer took 110 us of a short prompt's time)."""
     blk_t0, blk_n, seq_blk0, seq_nchunk, seq_t0, seq_len = [], [], [], [], [], []
     for i in range(len(cu_host) - 1):
         t0, n = cu_host[i], cu_host[i + 1] - cu_host[i]
@@ -1735,18 +1736,18 @@ def gdn_chunk_plan(cu_host, device):
         for b in range(0, n, 128):
             blk_t0.append(t0 + b)
             blk_n.append(min(128, n - b))
-    i32 = dict(dtype=torch.int32, device=device)
-    return tuple(torch.tensor(v, **i32) for v in (blk_t0, blk_n, seq_blk0, seq_nchunk, seq_t0, seq_len))
+    parts = (blk_t0, blk_n, seq_blk0, seq_nchunk, seq_t0, seq_len)
+    return torch.tensor([v for p in parts for v in p], dtype=torch.int32).to(device).split([len(p) for p in parts])
 
 
 def gdn_chunked(qkv, g, beta, state, cu_host, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps=1e-6,
-                write_state=True, out=None):
+                write_state=True, out=None, plan=None):
     """Gated delta rule over prompt-sized rows on the tensor cores (64-token chunks, ``csrc/gdn_chunk_sm100.cu``).
-    ``cu_host``: the sequence boundaries as a Python list. Heads of 128 x 128 only."""
+    ``cu_host``: the sequence boundaries as a Python list; ``plan``: their ``gdn_chunk_plan``. Heads of 128 x 128 only."""
     C = ext()
     T = qkv.shape[0]
     ws = Workspace.get(qkv.device)
-    blk_t0, blk_n, seq_blk0, seq_nchunk, seq_t0, seq_len = gdn_chunk_plan(cu_host, qkv.device)
+    blk_t0, blk_n, seq_blk0, seq_nchunk, seq_t0, seq_len = plan or gdn_chunk_plan(cu_host, qkv.device)
     nb = int(blk_t0.numel())
     need = C.gdn_chunk_scratch_bytes(nb, n_v)
     scratch = ws._cache.get("gdn_chunk_scratch")
@@ -1761,7 +1762,9 @@ def gdn_chunked(qkv, g, beta, state, cu_host, slots, n_k, n_v, dk, dv, tiled_hea
 
 
 def gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps=1e-6,
-                  write_state=True, out=None, cu_host=None):
+                  write_state=True, out=None, cu_host=None, step=None):
+    """``step``: an object with a ``gdn_plan`` attribute that keeps the chunk tables for the step's other layers; its sequence
+    boundaries are ``cu_host``."""
     C = ext()
     T = qkv.shape[0]
     # prompt chunks (many rows per sequence): the chunked tensor-core scan when the heads are 128 x 128, else the
@@ -1770,8 +1773,13 @@ def gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_he
     if prompt_rows and dk == 128 and dv == 128 and T >= 64 and TUNE["gdn_chunk"] and qkv.stride(0) % 8 == 0:
         if cu_host is None:
             cu_host = cu_seq.tolist()
+        plan = step.gdn_plan if step is not None else None
+        if plan is None:
+            plan = gdn_chunk_plan(cu_host, qkv.device)
+            if step is not None:
+                step.gdn_plan = plan
         return gdn_chunked(qkv, g, beta, state, cu_host, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps,
-                           write_state, out)
+                           write_state, out, plan)
     if out is None:
         out = torch.empty(T, n_v, dv, dtype=torch.bfloat16, device=qkv.device)
     C.gdn_recurrent(qkv, g, beta, state, cu_seq, slots, n_k, n_v, dk, dv, tiled_heads, scale, l2_eps, out,
