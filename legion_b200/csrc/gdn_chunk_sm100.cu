@@ -355,7 +355,12 @@ constexpr int SC_U = CH * D * 2;        // U chunk tile (plain rows)
 constexpr int SC_STAGE = 3 * SC_W + SC_M + SC_U;          // 73728
 constexpr int SC_SMEM = 2 * HALF_BYTES + HALF_BYTES + 2 * SC_STAGE + 1024 + 256;
 
-__global__ void __launch_bounds__(160, 1)
+// Bound by the chain of a chunk: state operand -> W S -> D -> new state, each step a product and a pass of the worker warps from
+// tensor memory to the next operand. What the chain does not need runs beside it: Q' S and M D (of which only the outputs
+// depend, two accumulators), the outputs of a chunk while the next one's W S is multiplied, the decays a chunk ahead. Two
+// threads share a row of the state. 8192 tokens of one sequence, 32 heads: 606 us with the outputs inside the chain and
+// one thread per row, 366 us now.
+__global__ void __launch_bounds__(288, 1)
 gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQg,
                       const __grid_constant__ CUtensorMap tmKd, const __grid_constant__ CUtensorMap tmM,
                       const __grid_constant__ CUtensorMap tmU, const ScanArgs a) {
@@ -366,11 +371,12 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   uint8_t* stg = d_a + HALF_BYTES;              // [2] x {W, Q', K', M, U}
   uint64_t* bars = reinterpret_cast<uint64_t*>(stg + 2 * SC_STAGE);
   uint64_t* ld_full = bars;        // [2]
-  uint64_t* s_ready = bars + 2;    // state operand + scaled accumulator ready (128 arrivals)
-  uint64_t* d_done = bars + 3;     // W S0 and Q' S0 done
-  uint64_t* dl_ready = bars + 4;   // D^T written (128 arrivals)
-  uint64_t* o_done = bars + 5;     // M D and K'^T D done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+  uint64_t* s_ready = bars + 2;    // state operand + scaled accumulator ready (256 arrivals)
+  uint64_t* d_done = bars + 3;     // W S0 done
+  uint64_t* dl_ready = bars + 4;   // D^T written (256 arrivals)
+  uint64_t* s_done = bars + 5;     // K'^T D done
+  uint64_t* o_done = bars + 6;     // [2] Q' S0 + M D of even / odd chunks done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int h = blockIdx.x, seq = blockIdx.y;
@@ -380,26 +386,27 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
 
   if (threadIdx.x == 0) {
     mbar_init(&ld_full[0], 1); mbar_init(&ld_full[1], 1);
-    mbar_init(s_ready, 128); mbar_init(d_done, 1); mbar_init(dl_ready, 128); mbar_init(o_done, 1);
+    mbar_init(s_ready, 256); mbar_init(d_done, 1); mbar_init(dl_ready, 256); mbar_init(s_done, 1);
+    mbar_init(&o_done[0], 1); mbar_init(&o_done[1], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4) {
-    tmem_alloc(tmem_slot, 256);
+  if (warp == 8) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tm_d = tmem, tm_o = tmem + 64, tm_s = tmem + 128;
+  const uint32_t tm_d = tmem, tm_o = tmem + 64, tm_s = tmem + 256;      // (two output accumulators, 64 columns each)
   griddep_wait();
   griddep_launch();
   auto chunk_row = [&](int c) -> int {      // first row of chunk c in the [items * 128, .] scratch tensors
     return int((long(blk0 + (c >> 1)) * a.Hv + h) * 128 + (c & 1) * 64);
   };
 
-  if (warp == 4) {
+  if (warp == 8) {
     if (lane == 0 && nchunk > 0) {
       tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmQg); tma_prefetch_desc(&tmKd); tma_prefetch_desc(&tmM);
       tma_prefetch_desc(&tmU);
@@ -423,38 +430,45 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       bool ok = true;
       for (int c = 0; ok && c < nchunk; ++c) {
         const uint32_t st = smem_u32(stg + (c & 1) * SC_STAGE);
-        ok = mbar_wait(s_ready, c & 1, abort_flag);        // S operand of this chunk ready; other stage is free
+        ok = mbar_wait(s_ready, c & 1, abort_flag);        // S operand of this chunk ready
         if (!ok) break;
-        if (c + 1 < nchunk) load_chunk(c + 1);
+        if (c + 1 < nchunk) {                              // the other stage is free once its chunk's last product is done
+          if (c > 0) ok = mbar_wait(&o_done[(c - 1) & 1], ((c - 1) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          load_chunk(c + 1);
+        }
         ok = mbar_wait(&ld_full[c & 1], (c >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sa = smem_u32(s_a), da = smem_u32(d_a);
+        const uint32_t sa = smem_u32(s_a), da = smem_u32(d_a), to = tm_o + (c & 1) * 64;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint64_t adesc = umma_desc_k_sw128(sa + (k >> 2) * HALF_BYTES + (k & 3) * 32);
-          const uint32_t boff = (k >> 2) * (CH * 128) + (k & 3) * 32;
-          umma_f16(tm_d, adesc, umma_desc_k_sw128(st + boff), idesc_d, k ? 1u : 0u);
-          umma_f16(tm_o, adesc, umma_desc_k_sw128(st + SC_W + boff), idesc_d, k ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_f16(tm_d, umma_desc_k_sw128(sa + (k >> 2) * HALF_BYTES + (k & 3) * 32),
+                   umma_desc_k_sw128(st + (k >> 2) * (CH * 128) + (k & 3) * 32), idesc_d, k ? 1u : 0u);
         umma_commit(d_done);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          umma_f16(to, umma_desc_k_sw128(sa + (k >> 2) * HALF_BYTES + (k & 3) * 32),
+                   umma_desc_k_sw128(st + SC_W + (k >> 2) * (CH * 128) + (k & 3) * 32), idesc_d, k ? 1u : 0u);
         ok = mbar_wait(dl_ready, c & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t adesc = umma_desc_k_sw128(da + k * 32);
-          umma_f16(tm_o, adesc, umma_desc_k_sw128(st + 3 * SC_W + k * 32), idesc_d, 1u);
-          umma_f16(tm_s, adesc, umma_desc_mn_sw128(st + 2 * SC_W + k * 16 * 128, CH * 128, 1024), idesc_s, 1u);
-        }
-        umma_commit(o_done);
+        for (int k = 0; k < 4; ++k)
+          umma_f16(tm_s, umma_desc_k_sw128(da + k * 32), umma_desc_mn_sw128(st + 2 * SC_W + k * 16 * 128, CH * 128, 1024),
+                   idesc_s, 1u);
+        umma_commit(s_done);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_f16(to, umma_desc_k_sw128(da + k * 32), umma_desc_k_sw128(st + 3 * SC_W + k * 32), idesc_d, 1u);
+        umma_commit(&o_done[c & 1]);
       }
       if (!ok) { *abort_flag = 1; atomicCAS(a.status, 0, ST_TIMEOUT_FULL); }
     }
   } else if (nchunk > 0) {
-    // ------------------------------------------------------------------ workers: thread r = dv row r
-    const int r = threadIdx.x;
-    const uint32_t lane_off = uint32_t(warp * 32) << 16;
+    // ------------------------------------------------------------------ workers: threads r and r + 128 = dv row r, half of the
+    // tokens and state columns each
+    const int r = threadIdx.x & 127, hf = threadIdx.x >> 7;
+    const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
     const int slot = a.slots[seq];
     float* st_g = a.state + (long(slot) * a.Hv + h) * D * D;            // [dk][dv]
     const int seq_t0 = a.seq_t0[seq], seq_len = a.seq_len[seq];
@@ -480,7 +494,7 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     {
       const float dec0 = a.gC[(long(blk0) * a.Hv + h) * 2];
 #pragma unroll 1
-      for (int c0 = 0; c0 < D; c0 += 32) {
+      for (int c0 = hf * 64; c0 < hf * 64 + 64; c0 += 32) {
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = st_g[long(c0 + j) * D + r];
@@ -495,21 +509,23 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     for (int c = 0; c < nchunk; ++c) {
       const uint8_t* st = stg + (c & 1) * SC_STAGE;
       const __nv_bfloat16* u_s = reinterpret_cast<const __nv_bfloat16*>(st + 3 * SC_W + SC_M);   // [64 tok][128 dv]
+      const bool last = c + 1 == nchunk;
+      const float dec_next = last ? 1.f : a.gC[(long(blk0 + ((c + 1) >> 1)) * a.Hv + h) * 2 + ((c + 1) & 1)];
       // ---- D^T = U^T - (W S0)^T
       if (ok) ok = mbar_wait(d_done, c & 1, abort_flag);
       tc_fence_after();
-#pragma unroll 1
-      for (int c0 = 0; c0 < CH; c0 += 32) {
+      {
+        const int c0 = hf * 32;
         uint32_t rr[32];
         tmem_ld32(tm_d + lane_off + c0, rr);
+        float u[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) u[j] = __bfloat162float(u_s[(c0 + j) * D + r]);
         tmem_ld_wait();
         uint32_t packed[16];
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float d0 = __bfloat162float(u_s[(c0 + j) * D + r]) - __uint_as_float(rr[j]);
-          const float d1 = __bfloat162float(u_s[(c0 + j + 1) * D + r]) - __uint_as_float(rr[j + 1]);
-          packed[j / 2] = pack_bf16x2(d0, d1);
-        }
+        for (int j = 0; j < 32; j += 2)
+          packed[j / 2] = pack_bf16x2(u[j] - __uint_as_float(rr[j]), u[j + 1] - __uint_as_float(rr[j + 1]));
         uint8_t* base = d_a + r * 128;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -521,24 +537,11 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(dl_ready);
-      // ---- outputs of the chunk and the new state
-      if (ok) ok = mbar_wait(o_done, c & 1, abort_flag);
+      // ---- the new state
+      if (ok) ok = mbar_wait(s_done, c & 1, abort_flag);
       tc_fence_after();
-      const int tok0 = seq_t0 + c * CH;
-      const int nt = min(CH, seq_len - c * CH);
 #pragma unroll 1
-      for (int c0 = 0; c0 < CH; c0 += 32) {
-        uint32_t rr[32];
-        tmem_ld32(tm_o + lane_off + c0, rr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < nt) a.out[(long(tok0 + c0 + j) * a.Hv + h) * D + r] = __float2bfloat16(__uint_as_float(rr[j]));
-      }
-      const bool last = c + 1 == nchunk;
-      const float dec_next = last ? 1.f : a.gC[(long(blk0 + ((c + 1) >> 1)) * a.Hv + h) * 2 + ((c + 1) & 1)];
-#pragma unroll 1
-      for (int c0 = 0; c0 < D; c0 += 32) {
+      for (int c0 = hf * 64; c0 < hf * 64 + 64; c0 += 32) {
         uint32_t rr[32];
         tmem_ld32(tm_s + lane_off + c0, rr);
         tmem_ld_wait();
@@ -560,14 +563,26 @@ gdn_chunk_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         tc_fence_before();
         mbar_arrive(s_ready);
       }
+      // ---- outputs, beside the next chunk's first product (the accumulator is multiplied into again two chunks on)
+      if (ok) ok = mbar_wait(&o_done[c & 1], (c >> 1) & 1, abort_flag);
+      tc_fence_after();
+      const int tok0 = seq_t0 + c * CH;
+      const int nt = min(CH, seq_len - c * CH);
+      uint32_t rr[32];
+      tmem_ld32(tm_o + (c & 1) * 64 + lane_off + hf * 32, rr);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (hf * 32 + j < nt) a.out[(long(tok0 + hf * 32 + j) * a.Hv + h) * D + r] = __float2bfloat16(__uint_as_float(rr[j]));
+      tc_fence_before();
     }
     if (!ok) { *abort_flag = 1; atomicCAS(a.status, 0, ST_TIMEOUT_TMEM_FULL); }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == 8) {
     tc_fence_after();
-    tmem_dealloc(tmem, 256);
+    tmem_dealloc(tmem, 512);
   }
 }
 
@@ -617,7 +632,7 @@ int gdn_chunk_launch(const void* qkv, long ld, long T, const float* g, const flo
   sa.seq_blk0 = seq_blk0; sa.seq_nchunk = seq_nchunk; sa.seq_t0 = seq_t0; sa.seq_len = seq_len; sa.slots = slots;
   sa.gC = pa.gC; sa.state = state; sa.out = static_cast<__nv_bfloat16*>(out); sa.Hv = Hv; sa.write_state = write_state;
   sa.status = status;
-  launch_pdl(gdn_chunk_scan_kernel, dim3(Hv, n_seqs), dim3(160), SC_SMEM, s, *tmW, *tmQg, *tmKd, *tmM, *tmU, sa);
+  launch_pdl(gdn_chunk_scan_kernel, dim3(Hv, n_seqs), dim3(288), SC_SMEM, s, *tmW, *tmQg, *tmKd, *tmM, *tmU, sa);
   return cudaGetLastError() != cudaSuccess;
 }
 
