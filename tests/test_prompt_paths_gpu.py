@@ -119,7 +119,7 @@ def test_short_prompt_gemm(T, N, K):
 
 # pairs of 256 query rows: one row more than a tile, an empty second tile, full pairs, short sequences beside long ones, cached
 # tokens in front; blocks of 128 keys with a remainder; head sizes between and at the kernel's, pages of a part of its tiles
-@pytest.mark.parametrize("q_lens,cached,page", [([129], 0, 64), ([256, 1, 130], 70, 16), ([257, 511], 128, 32), ([700, 128], 333, 64)])
+@pytest.mark.parametrize("q_lens,cached,page", [([129], 0, 64), ([256, 1, 130], 70, 16), ([257, 511], 128, 32), ([1100, 128], 333, 64)])
 @pytest.mark.parametrize("Hq,Hkv,dk,dv", [(4, 2, 128, 128), (2, 2, 192, 128), (8, 1, 256, 256), (2, 1, 136, 72), (2, 1, 232, 208)])
 def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
     n, T = len(q_lens), sum(q_lens)
@@ -141,3 +141,42 @@ def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
         # bf16 probabilities and output, 2^-9 each; single rows up to 2^-6 of the largest value
         assert (out[a:b].double() - want).norm() < 2.0 ** -8 * want.norm()
         assert (out[a:b].double() - want).abs().max() < 2.0 ** -6 * want.abs().max()
+
+
+# eight columns per thread and, where rows do not lie on 16 bytes, one: head sizes, partial and whole rotation, a query gate,
+# a token without a cell, a last warp that is not full
+@pytest.mark.parametrize("T,Hq,Hkv,D,rot,gated,shift", [(5, 3, 1, 64, 64, False, 0), (130, 4, 2, 128, 128, False, 0), (33, 2, 1, 256, 64, True, 0),
+                                                        (7, 5, 3, 128, 0, False, 0), (9, 3, 1, 128, 64, True, 1)])
+def test_qk_prep_and_gate(T, Hq, Hkv, D, rot, gated, shift):
+    from legion_b200.ops import reference as ref
+    S = D * (2 if gated else 1)
+    wide = Hq * S + 2 * Hkv * D
+    qkv = _rnd(T, wide + shift)[:, shift:]
+    qw, kw = (1 + 0.1 * torch.randn(D, generator=torch.Generator().manual_seed(i)).to(DEV) for i in (1, 2))
+    cs = ref.rope_cos_sin(512, max(rot, 64), 1e4, None, device=DEV)
+    pos = torch.randint(0, 512, (T,), generator=torch.Generator().manual_seed(3)).int().to(DEV)
+    slots = torch.randperm(4 * 64, generator=torch.Generator().manual_seed(4))[:T].to(DEV)
+    slots[T // 2] = -1
+    kc, vc = torch.zeros(4, 64, Hkv, D, dtype=torch.bfloat16, device=DEV), torch.zeros(4, 64, Hkv, D, dtype=torch.bfloat16, device=DEV)
+    out = sm().qk_norm_rope_append(qkv, Hq, Hkv, D, qw, kw, 1e-6, 0.0, cs, rot, pos, slots, kc, vc, gated)
+    x = qkv.double()
+    heads = x[:, :Hq * S].view(T, Hq, S)
+
+    def prep(v, w):
+        v = v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        if rot:
+            c, s = cs[pos.long()].double()[:, None, :rot].chunk(2, -1)
+            a, b = v[..., :rot // 2].clone(), v[..., rot // 2:rot].clone()
+            v = torch.cat([a * c - b * s, b * c + a * s, v[..., rot:]], -1)
+        return v
+    # one bf16 rounding of fp32 values
+    close = lambda a, b: ((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 1e-5).all()       # noqa: E731
+    assert close(out, prep(heads[..., :D], qw))
+    live = slots >= 0
+    k = prep(x[:, Hq * S:Hq * S + Hkv * D].view(T, Hkv, D), kw)
+    assert close(kc.view(-1, Hkv, D)[slots[live]], k[live])
+    assert torch.equal(vc.view(-1, Hkv, D)[slots[live]].double(), x[:, Hq * S + Hkv * D:].view(T, Hkv, D)[live])
+    assert int((kc.view(-1, Hkv * D).abs().sum(-1) > 0).sum()) == T - 1
+    if gated:
+        o = sm().sigmoid_gate(out, qkv, Hq, D)
+        assert close(o.view(T, Hq, D), out.double() * torch.sigmoid(heads[..., D:]))
