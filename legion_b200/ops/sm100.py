@@ -1093,9 +1093,17 @@ def latent_prompt(q, kv, gate, uk_rows, uv, norm_w, eps, cos_sin, cache, p: Late
     return o
 
 
+MLA_EXPAND_FREE = 512 << 20      # expanded keys and values of a step may always take this much
+
+
 def mla_expand_ok(q, kv_b, cache, p: LatentPart, heads: int, dim: int, rot: int, vdim: int, rank: int) -> bool:
-    return (latent_expand_ok(q, cache, p, heads, dim, rot, rot, rank, vdim) and q.is_contiguous() and tma_ok(kv_b)
-            and kv_b.is_contiguous() and vdim % 64 == 0)
+    """Whether a step's long portions attend per head: sizes the kernels take, and no more scratch than the latent form's query
+    and output rows would need (a short portion behind a long history stays in the latent space for that)."""
+    if not (latent_expand_ok(q, cache, p, heads, dim, rot, rot, rank, vdim) and q.is_contiguous() and tma_ok(kv_b)
+            and kv_b.is_contiguous() and vdim % 64 == 0):
+        return False
+    scratch = p.pages.shape[1] * 64 * (heads * (dim + rot + vdim) + rank) * 2
+    return scratch <= max(MLA_EXPAND_FREE, q.shape[0] * heads * (2 * rank + rot) * 2)
 
 
 def mla_prompt(q, kv_b, cache, p: LatentPart, scale, heads: int, dim: int, rot: int, rank: int):
