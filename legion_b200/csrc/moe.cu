@@ -583,17 +583,14 @@ int moe_route_small_launch(const void* x, long ldx, const float* norm_w, float e
   auto xn = static_cast<__nv_bfloat16*>(x_normed);
   auto wb = static_cast<const __nv_bfloat16*>(w);
   const int epc = E >= 256 ? 8 : 4;                              // router rows per CTA
-  // the columns are split over CTAs too, so that the weight stream and the staging of the token rows spread over more SMs
-  // (the logit and gate buffers hold ROUTE_MAX_KSPLIT planes): wide models always, others as long as every CTA has an SM.
-  // 512 experts, width 2048, 64 / 16 / 1 tokens: 42 / 18 / 13 us with whole rows, 32 / 15 / 12 with halves of them
-  const int groups = (E + (sh_gate_w ? 1 : 0) + epc - 1) / epc;
-  int ksplit = ROUTE_MAX_KSPLIT;
-  while (ksplit > 1 && ((H / 8) % ksplit || (H < 4096 && (groups * ksplit > 148 || H / ksplit < 512)))) ksplit /= 2;
+  // wide models: the columns are split over CTAs too, so that the weight stream and the staging of the token rows
+  // spread over four times as many SMs (the logit and gate buffers hold ROUTE_MAX_KSPLIT planes)
+  const int ksplit = (H >= 4096 && (H / 8) % ROUTE_MAX_KSPLIT == 0) ? ROUTE_MAX_KSPLIT : 1;
   const int Hs = H / ksplit;
   const int tpp = size_t(16) * Hs * 2 <= 192 * 1024 ? 16 : 8;    // tokens staged per pass
   if (size_t(tpp) * Hs * 2 > 200 * 1024) return 1;
   const int smem = tpp * Hs * 2;
-  const int grid = groups * ksplit;
+  const int grid = ((E + (sh_gate_w ? 1 : 0) + epc - 1) / epc) * ksplit;
 #define LB_ROUTE(MAXE, EXT)                                                                                         \
   {                                                                                                                 \
     static int smem_set = 0;                                                                                        \
