@@ -191,81 +191,11 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
     v[2 * j + 1] = f.y;
   }
 }
-__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
-  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
   uint4 u;
   u.x = pack_bf16x2(v[0], v[1]); u.y = pack_bf16x2(v[2], v[3]);
   u.z = pack_bf16x2(v[4], v[5]); u.w = pack_bf16x2(v[6], v[7]);
   *reinterpret_cast<uint4*>(p) = u;
-}
-
-// The same with eight neighbouring columns per thread, D / 8 threads per head, for rows that lie on 16 bytes: bound by the
-// memory's bandwidth instead of by the number of two-byte accesses (5500 tokens, 40 heads of 128: 66 -> 42 us). A column's rotation partner is half / 8
-// lanes away.
-template <int D>
-__global__ void __launch_bounds__(128) qk_norm_rope_append8_kernel(
-    const __nv_bfloat16* __restrict__ qkv, long ld_qkv, int q_head_stride, int k_off, int v_off,
-    const float* __restrict__ qw, const float* __restrict__ kw, float eps, float w_offset,
-    const float* __restrict__ cos_sin, int rot, const int* __restrict__ positions, const long* __restrict__ slots,
-    __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
-    long cache_cell_stride, int T, int Hq, int Hkv) {
-  constexpr int LPH = D / 8;
-  griddep_wait();
-  griddep_launch();
-  const unsigned heads = Hq + 2 * Hkv;
-  const unsigned g = (blockIdx.x * 128u + threadIdx.x) / LPH;
-  const bool live = g < unsigned(T) * heads;                       // (whole warps stay for the shuffles)
-  const int t = live ? int(g / heads) : 0, h = live ? int(g - unsigned(t) * heads) : 0;
-  const int i = (threadIdx.x % LPH) * 8;
-  const int kind = h < Hq ? 0 : (h < Hq + Hkv ? 1 : 2);
-  const __nv_bfloat16* src = qkv + t * ld_qkv + (kind == 0 ? long(h) * q_head_stride
-                                                           : (kind == 1 ? k_off + long(h - Hq) * D : v_off + long(h - Hq - Hkv) * D));
-  float v[8];
-  load8(src + i, v);
-  const float* nw = kind == 0 ? qw : (kind == 1 ? kw : nullptr);
-  float ss = 0.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
-#pragma unroll
-  for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if (nw) {
-    const float inv = rsqrtf(ss / float(D) + eps);
-    float w[8];
-    load8(nw + i, w);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = v[j] * inv * (w[j] + w_offset);
-  }
-  if (rot > 0) {
-    const int half = rot / 2;
-    const bool low = i < half, turns = kind != 2 && i < rot;
-    float p[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float up = __shfl_down_sync(0xffffffffu, v[j], half / 8), down = __shfl_up_sync(0xffffffffu, v[j], half / 8);
-      p[j] = low ? up : down;
-    }
-    if (turns) {
-      const float* cs = cos_sin + long(positions[t]) * rot + (low ? i : i - half);
-      float c[8], s[8];
-      load8(cs, c);
-      load8(cs + half, s);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = low ? v[j] * c[j] - p[j] * s[j] : v[j] * c[j] + p[j] * s[j];
-    }
-  }
-  if (!live) return;
-  if (kind == 0) {
-    store8(q_out + (long(t) * Hq + h) * D + i, v);
-    return;
-  }
-  const long cell = slots[t];
-  if (cell < 0) return;
-  __nv_bfloat16* base = kind == 1 ? k_cache : v_cache;
-  store8(base + cell * cache_cell_stride + long(h - Hq - (kind == 1 ? 0 : Hkv)) * D + i, v);
 }
 
 int qk_norm_rope_append_launch(const void* qkv, long ld_qkv, int q_head_stride, int k_off, int v_off, const float* qw,
@@ -274,22 +204,6 @@ int qk_norm_rope_append_launch(const void* qkv, long ld_qkv, int q_head_stride, 
                                long cache_cell_stride, int T, int Hq, int Hkv, int D, cudaStream_t s) {
   if (T <= 0) return 0;
   if (rot % 64 != 0 || rot > D) return 1;
-  auto on16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  if (on16(qkv) && on16(q_out) && on16(k_cache) && on16(v_cache) && on16(qw) && on16(kw) && on16(cos_sin) && ld_qkv % 8 == 0 &&
-      q_head_stride % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && cache_cell_stride % 8 == 0 &&
-      long(T) * (Hq + 2 * Hkv) < (1L << 26)) {
-    const unsigned vec_blocks = unsigned((long(T) * (Hq + 2 * Hkv) * (D / 8) + 127) / 128);
-#define LB_D(DD)                                                                                                   \
-  if (D == DD) {                                                                                                   \
-    return launch_pdl(qk_norm_rope_append8_kernel<DD>, dim3(vec_blocks), dim3(128), 0, s,                         \
-                      static_cast<const __nv_bfloat16*>(qkv), ld_qkv, q_head_stride, k_off, v_off, qw, kw, eps,    \
-                      w_offset, cos_sin, rot, positions, slots, static_cast<__nv_bfloat16*>(q_out),                \
-                      static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache),                  \
-                      cache_cell_stride, T, Hq, Hkv) != cudaSuccess;                                               \
-  }
-    LB_D(64) LB_D(128) LB_D(256)
-#undef LB_D
-  }
   const long warps = long(T) * (Hq + 2 * Hkv);
   const int blocks = int((warps * 32 + 127) / 128);
 #define LB_D(DD)                                                                                                   \

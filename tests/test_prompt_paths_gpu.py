@@ -143,7 +143,7 @@ def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
         assert (out[a:b].double() - want).abs().max() < 2.0 ** -6 * want.abs().max()
 
 
-# eight columns per thread and, where rows do not lie on 16 bytes, one: head sizes, partial and whole rotation, a query gate,
+# query and key preparation and the gate (eight columns per thread, one where rows do not lie on 16 bytes): partial and whole rotation,
 # a token without a cell, a last warp that is not full
 @pytest.mark.parametrize("T,Hq,Hkv,D,rot,gated,shift", [(5, 3, 1, 64, 64, False, 0), (130, 4, 2, 128, 128, False, 0), (33, 2, 1, 256, 64, True, 0),
                                                         (7, 5, 3, 128, 0, False, 0), (9, 3, 1, 128, 64, True, 1)])
