@@ -326,32 +326,39 @@ __global__ void __launch_bounds__(THREADS) gdn_decode_fused_kernel(
   const float bt = 1.f / (1.f + __expf(-__bfloat162float(row[C + Hv * DV + h])));
   __syncthreads();
   const float qn = qn_s, kn = kn_s;
-  float kv = 0.f;
+  // sums over the key dimension run in two chains of DK / 2 cells: with four threads per column, the odd ones go on from the
+  // even ones' sums (a barrier more each; the results do not depend on the number of threads)
+  auto chain = [&](const float* x, float f) {
+    float v = 0.f;
+    if (NS == 4) {
+      if (!(part_i & 1)) {
 #pragma unroll
-  for (int i = 0; i < CELLS; ++i) kv += S[i] * k_s[part_i * CELLS + i];
-  part[j][part_i][c] = kv * kn;
-  __syncthreads();
-  auto sum = [&]() {
-    float v = part[j][0][c] + part[j][1][c];
-    if constexpr (NS == 4) v += part[j][2][c] + part[j][3][c];
-    return v;
+        for (int i = 0; i < CELLS; ++i) v += S[i] * x[part_i * CELLS + i];
+        part[j][part_i][c] = v;
+      }
+      __syncthreads();
+      if (part_i & 1) v = part[j][part_i - 1][c];
+    }
+    if (NS == 2 || (part_i & 1)) {
+#pragma unroll
+      for (int i = 0; i < CELLS; ++i) v += S[i] * x[part_i * CELLS + i];
+      part[j][part_i][c] = v * f;
+    }
+    __syncthreads();
+    return NS == 4 ? part[j][1][c] + part[j][NS - 1][c] : part[j][0][c] + part[j][1][c];
   };
-  const float delta = (v_s[j][c] - gt * sum()) * bt;
+  const float delta = (v_s[j][c] - gt * chain(k_s, kn)) * bt;
   __syncthreads();
-  float o = 0.f;
 #pragma unroll
   for (int i = 0; i < CELLS; ++i) {
     S[i] = gt * S[i] + k_s[part_i * CELLS + i] * kn * delta;
-    o += S[i] * q_s[part_i * CELLS + i];
+    sp[long(i) * DV] = S[i];
   }
-  part[j][part_i][c] = o * qn;
-#pragma unroll
-  for (int i = 0; i < CELLS; ++i) sp[long(i) * DV] = S[i];
-  __syncthreads();
+  const float o = chain(q_s, qn);
   // gated RMS norm over the head's DV outputs
   float ov = 0.f, ss = 0.f;
   if (part_i == 0) {
-    ov = __bfloat162float(__float2bfloat16(sum()));
+    ov = __bfloat162float(__float2bfloat16(o));
     ss = ov * ov;
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
@@ -442,62 +449,10 @@ __global__ void __launch_bounds__(128) gated_rmsnorm_kernel(const __nv_bfloat16*
   }
 }
 
-// eight neighbouring columns per thread, DV / 8 threads per row (rows on 16 bytes). 8192 tokens, 32 heads: 69 -> 38 us
-template <int DV>
-__global__ void __launch_bounds__(128) gated_rmsnorm8_kernel(const __nv_bfloat16* __restrict__ o,
-                                                             const __nv_bfloat16* __restrict__ z, long ldz,
-                                                             const float* __restrict__ w, float eps, int Hv, unsigned n_rows,
-                                                             int act, __nv_bfloat16* __restrict__ out) {
-  constexpr int LPR = DV / 8;
-  const unsigned r = (blockIdx.x * 128u + threadIdx.x) / LPR;
-  const bool live = r < n_rows;                                    // (whole warps stay for the shuffles)
-  const unsigned t = live ? r / unsigned(Hv) : 0u, h = live ? r - t * unsigned(Hv) : 0u;
-  const int i = (threadIdx.x % LPR) * 8;
-  const uint4 uo = *reinterpret_cast<const uint4*>(o + long(live ? r : 0u) * DV + i);
-  const uint4 uz = *reinterpret_cast<const uint4*>(z + t * ldz + long(h) * DV + i);
-  const __nv_bfloat162 *ho = reinterpret_cast<const __nv_bfloat162*>(&uo), *hz = reinterpret_cast<const __nv_bfloat162*>(&uz);
-  float v[8], ss = 0.f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = __bfloat1622float2(ho[j]);
-    v[2 * j] = f.x;
-    v[2 * j + 1] = f.y;
-    ss += f.x * f.x + f.y * f.y;
-  }
-#pragma unroll
-  for (int k = LPR / 2; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
-  if (!live) return;
-  const float inv = rsqrtf(ss / float(DV) + eps);
-  const float4 w0 = reinterpret_cast<const float4*>(w + i)[0], w1 = reinterpret_cast<const float4*>(w + i)[1];
-  const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-  uint4 u;
-  __nv_bfloat162* hu = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 zf = __bfloat1622float2(hz[j]);
-    const float s0 = 1.f / (1.f + __expf(-zf.x)), s1 = 1.f / (1.f + __expf(-zf.y));
-    hu[j] = __floats2bfloat162_rn(v[2 * j] * inv * wv[2 * j] * (act == 0 ? zf.x * s0 : s0),
-                                  v[2 * j + 1] * inv * wv[2 * j + 1] * (act == 0 ? zf.y * s1 : s1));
-  }
-  *reinterpret_cast<uint4*>(out + long(r) * DV + i) = u;
-}
-
 int gated_rmsnorm_launch(const void* o, const void* z, long ldz, const float* w, float eps, int DV, int Hv, long T,
                          int act, void* out, cudaStream_t s) {
   const long rows = T * Hv;
   if (rows <= 0) return 0;
-  if (((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w) |
-        reinterpret_cast<uintptr_t>(out)) & 15) == 0 && ldz % 8 == 0 && rows < (1L << 26)) {
-#define LB_GN(D_)                                                                                                     \
-  if (DV == D_) {                                                                                                     \
-    gated_rmsnorm8_kernel<D_><<<unsigned((rows * (D_ / 8) + 127) / 128), 128, 0, s>>>(                                \
-        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(z), ldz, w, eps, Hv, unsigned(rows),  \
-        act, static_cast<__nv_bfloat16*>(out));                                                                       \
-    return cudaGetLastError() != cudaSuccess;                                                                         \
-  }
-    LB_GN(64) LB_GN(128) LB_GN(256)
-#undef LB_GN
-  }
   gated_rmsnorm_kernel<<<int((rows * 32 + 127) / 128), 128, 0, s>>>(static_cast<const __nv_bfloat16*>(o),
                                                                     static_cast<const __nv_bfloat16*>(z), ldz, w, eps,
                                                                     DV, Hv, rows, act,
