@@ -523,13 +523,17 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
     }
     const float ll = s_l[q];
-    float f = ll > 0.f ? 1.f / ll : 0.f;
+    float f = 1.f;
     __nv_bfloat16* dst = a.out + (long(b) * a.Hq + head0 + q) * D + d;
     if constexpr (EXT) {
-      f *= x.out_scale;
+      f = ll > 0.f ? x.out_scale / ll : 0.f;
       if (x.gate)
         f /= 1.f + __expf(-__bfloat162float(static_cast<const __nv_bfloat16*>(x.gate)[b * x.ld_gate + head0 + q]));
       dst = a.out + b * x.ldo + (head0 + q) * D + d;
+    }
+    if constexpr (!EXT) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = ll > 0.f ? o[i] / ll : 0.f;
     }
     if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
       uint2 u;

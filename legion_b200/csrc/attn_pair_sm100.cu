@@ -43,7 +43,7 @@ struct PairAttnCfg {
   static constexpr int VS = DV == 256 ? 3 : 4;
   static constexpr int KS = (222 * 1024 - Q_BYTES - VS * V_BYTES) / K_BYTES >= 4 ? 4 : (DK == 256 && DV == 256 ? 2 : 3);
   static constexpr int RING = Q_BYTES + KS * K_BYTES + VS * V_BYTES;
-  static constexpr int SMEM = RING + 2 * 2 * 128 * 4 + 512;
+  static constexpr int SMEM = RING + (2 * 2 + 1) * 128 * 4 + 512;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
 };
 
@@ -102,7 +102,8 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* k_s = q_s + Cfg::Q_BYTES;
   uint8_t* v_s = k_s + KS * Cfg::K_BYTES;
   float* mxs = reinterpret_cast<float*>(smem + Cfg::RING);       // [parity][warpgroup][row]
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(mxs + 2 * 2 * 128);
+  float* sums = mxs + 2 * 2 * 128;                               // [row], of the second warpgroup's keys
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sums + 128);
   uint64_t* k_full = q_full + 1;       // [4]  counted in the first CTA, as q_full, v_full and p_ready
   uint64_t* k_empty = k_full + 4;      // [4]  in both, as the rest
   uint64_t* v_full = k_empty + 4;      // [4]
@@ -248,7 +249,9 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int hi = row < rows_here ? min(ctx, qpos + 1) : 0;                  // keys that the row sees
     constexpr int OC = DV / 2;
     const uint32_t my_O = tmem_O + lane_off + wg * OC;
-    float m = -INFINITY, l = 0.f;
+    float m = -INFINITY, l = 0.f, alpha = 1.f, sum = 0.f;
+    // the first warpgroup adds both halves of the block before to the row's sum, in the order of the keys
+    auto add_sums = [&]() { l = l * alpha + sum; l += sums[row]; };
     bool ok = true;
     auto fail = [&](int code) { *abort_flag = 1; atomicCAS(a.status, 0, code | SITE_PREFILL_ATTN); ok = false; };
     for (int i = 0; i < n_blk; ++i) {
@@ -279,19 +282,28 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int j = 0; j < 64; ++j)
           if (key0 + j < hi) mx = fmaxf(mx, __uint_as_float(r[j]));
       }
-      // the other half's maximum; past this barrier the scores have been read and P may go over them
+      // both halves' maxima; past this barrier the scores have been read and P may go over them
       float* ex = mxs + (i & 1) * 256;
       ex[wg * 128 + row] = mx;
       tc_fence_before();
       asm volatile("bar.sync 1, 256;" ::: "memory");
       tc_fence_after();
-      mx = fmaxf(mx, ex[(wg ^ 1) * 128 + row]);
-      const float m_blk = mx * a.scale_log2;
-      float alpha = 1.f, sum;
-      if (m_blk > m + RESCALE_LOG2 || (m == -INFINITY && m_blk != -INFINITY)) {
-        alpha = (m == -INFINITY) ? 0.f : exp2f(m - m_blk);
-        m = m_blk;
+      const float other = ex[(wg ^ 1) * 128 + row];
+      if (i >= 1 && wg == 0) {
+        add_sums();
+        asm volatile("bar.arrive 2, 256;" ::: "memory");
       }
+      alpha = 1.f;
+      // the reference moves as it would over blocks of 64 keys, so that the probabilities are rounded as the single CTA's are
+      auto follow = [&](float half) {
+        const float h = half * a.scale_log2;
+        if (h > m + RESCALE_LOG2 || (m == -INFINITY && h != -INFINITY)) {
+          alpha = (m == -INFINITY) ? 0.f : alpha * exp2f(m - h);
+          m = h;
+        }
+      };
+      follow(wg == 0 ? mx : other);
+      follow(wg == 0 ? other : mx);
       const float neg_m = (m == -INFINITY) ? 0.f : -m;
       uint32_t packed[32];
       if (inner) {
@@ -327,7 +339,10 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           packed[j / 2] = *reinterpret_cast<const uint32_t*>(&b);
         }
       }
-      l = l * alpha + sum;
+      if (wg == 1) {
+        if (i >= 1) asm volatile("bar.sync 2, 256;" ::: "memory");      // the sum before this one has been read
+        sums[row] = sum;
+      }
       if (ok) {
         // cell c of the row holds keys 2 c (low half) and 2 c + 1
         st16(S + wg * 32, &packed[0]);
@@ -358,11 +373,13 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (ok && n_blk > 0 &&
         !__all_sync(0xffffffffu, mbar_wait(&o_done[(n_blk - 1) & 1], uint32_t((n_blk - 1) >> 1) & 1u, abort_flag)))
       fail(ST_TIMEOUT_TMEM_FULL);
-    // row sums of both halves (the exchange area of the parity that the last block did not use)
-    float* ex = mxs + (n_blk & 1) * 256;
-    ex[wg * 128 + row] = l;
     asm volatile("bar.sync 1, 256;" ::: "memory");
-    l += ex[(wg ^ 1) * 128 + row];
+    if (wg == 0) {
+      if (n_blk > 0) add_sums();
+      mxs[row] = l;                    // (past the barrier nobody reads maxima)
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    l = mxs[row];
     if (ok) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
