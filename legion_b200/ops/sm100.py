@@ -475,29 +475,31 @@ def pick_bn(n_tok: int, dual: bool) -> int:
 @functools.lru_cache(maxsize=4096)
 def _pick_tile(T: int, n_feat: int, K: int, dual: bool):
     """(token tile, K splits) of a bf16 GEMM with more than 32 tokens that does not fill the pairs of SMs
-    (``gemm_pair_sm100.cu``): the pair with the least modelled time, in cycles. A k block of 64 costs what its operands move
-    through shared memory in and out at 128 bytes per cycle, 32 columns of accumulators about 1400 cycles on their way out; a
-    split adds its partial sums. Short prompts otherwise ran as one wide token tile on a few SMs, or with their sums spread
-    over so many splits that adding those up took most of the time: 217 tokens, 2048 x 4096 weights, 34 us with 256-token
-    tiles in nine splits, 12 us with 64-token tiles in two."""
+    (``gemm_pair_sm100.cu``). The splits are those of the widest token tile, so that the sums, and with them the 4-bit
+    activations behind them, do not depend on the tile; the tile is the one with the least modelled time, in cycles. A k block of
+    64 costs what its operands move through shared memory in and out at 128 bytes per cycle, 32 columns of accumulators about
+    1400 cycles on their way out; a split adds its partial sums. With the widest tile short prompts ran on a few SMs, whose last
+    CTAs added up to nine partial sums of 256 tokens each."""
     ft, nw, num_kb = (n_feat + 127) // 128, 2 if dual else 1, (K + 63) // 64
+    wide = pick_bn(T, dual)
+    n_tt = (T + wide - 1) // wide
+    sk = _pick_split_k(n_tt, ft, K)
+    if n_tt * ft * sk * wide * nw * 128 > SPLITK_FLOATS:
+        sk = 1
     if T > 128 and ((T + 255) // 256) * ((nw * n_feat + 255) // 256) >= NUM_SMS // 2 and K >= 512:
-        return (128 if dual else 256), 1
+        return (128 if dual else 256), sk
     best = None
     for bn in (32, 64, 128) if dual else (32, 64, 128, 256):
-        if bn > 32 and bn // 2 >= T:
-            continue
         tiles = ((T + bn - 1) // bn) * ft
-        for sk in (1, 2, 3, 4, 6, 8):
-            if sk > 1 and (num_kb < 4 * sk or tiles * sk > 2 * NUM_SMS or tiles * sk * bn * nw * 128 > SPLITK_FLOATS):
-                continue
-            waves, kbs = (tiles * sk + NUM_SMS - 1) // NUM_SMS, (num_kb + sk - 1) // sk
-            main = kbs * (16384 * nw + 128 * bn * nw + 16384 * nw + 128 * bn) // 128
-            out = bn // 32 * (1400 * nw if sk == 1 else nw * (700 + 500 * sk))
-            cost = 2500 + (waves * max(main, out) + min(main, out))
-            if best is None or cost < best[0]:
-                best = (cost, bn, sk)
-    return best[1], best[2]
+        if bn > wide or (sk > 1 and tiles * sk * bn * nw * 128 > SPLITK_FLOATS):
+            continue
+        waves, kbs = (tiles * sk + NUM_SMS - 1) // NUM_SMS, (num_kb + sk - 1) // sk
+        main = kbs * (16384 * nw + 128 * bn * nw + 16384 * nw + 128 * bn) // 128
+        out = bn // 32 * (1400 * nw if sk == 1 else nw * (700 + 500 * sk))
+        cost = 2500 + (waves * max(main, out) + min(main, out))
+        if best is None or cost < best[0]:
+            best = (cost, bn)
+    return best[1], sk
 
 
 def _pick_split_k(n_tok_tiles: int, feat_tiles: int, K: int) -> int:
