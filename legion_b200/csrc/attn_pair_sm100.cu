@@ -4,8 +4,8 @@
 // of the keys and half of the value columns, and the products of both read both halves. A CTA by itself, with 64 keys at
 // a time, moves twice the keys and values per row and reads its queries from shared memory twice as often: at head size 256
 // that is 192 KB through shared memory per 64 keys, 1500 cycles for 1024 cycles of products, and its four softmax warps
-// waited for one another's steps most of the time. 4096 tokens, single CTAs / pairs: 40 heads of 128 542 / 645 TFLOP/s, 16
-// heads of 256 435 / 917, 32 heads of 192 (values 128) 354 / 743. Bound now by the softmax (exponentials and its chain of
+// waited for one another's steps most of the time. 4096 tokens, single CTAs / pairs: 40 heads of 128 542 / 645 TFLOP/s, 32
+// heads of 192 (values 128) 354 / 743, before the row sums joined in the order of 64-key blocks. Bound now by the softmax (exponentials and its chain of
 // tensor-memory and barrier latencies), not by the products.
 //   warp 0, lane 0   TMA: queries and keys (both CTAs' copies are counted on the first CTA's barriers)
 //   warp 10, lane 0  TMA: values
