@@ -67,13 +67,25 @@ class DecodeGraphs:
         the 30B-A3B 1.69 / 1.80, 4 dense layers of width 5120 1.43 / 1.56, 6 of latent attention 1.36 / 1.48. Never two
         for ranks that take part in collectives (their order must be the same on every rank), for offloaded experts, and
         for models whose sublayers run on branches of their own (``Decoder._branch``)."""
+        return 2 if self._halves(B) and int(ops.sm100.TUNE.get("decode_lanes", 1)) >= 2 else 1
+
+    def _halves(self, B: int) -> bool:
+        """Whether a step of ``B`` rows may run as two halves."""
         eng = self.eng
-        pc = eng.model.pctx
         if eng.mcfg.parallel_sublayers and ops.sm100.TUNE["parallel_branches"]:
-            return 1
-        if B < 64 or B % 2 or getattr(pc, "world", 1) > 1 or eng.dp_world > 1 or eng.model.expert_cache:
-            return 1
-        return 2 if int(ops.sm100.TUNE.get("decode_lanes", 1)) >= 2 else 1
+            return False
+        return not (B < 64 or B % 2 or getattr(eng.model.pctx, "world", 1) > 1 or eng.dp_world > 1 or eng.model.expert_cache)
+
+    def _holds(self, kind) -> bool:
+        return any(isinstance(t, kind) for t in self.eng.model.w.values())
+
+    def _split_seqs(self, B: int) -> int:
+        """Sequences that the key splits of the attention are planned for. The number of splits decides the order of the sums;
+        where 4-bit activations follow, which make 3% of the logits of another order, it is the same for a step that may run as
+        two halves in one lane and in two: that of a half (64 users of the 80B-A3B shape, 1500 tokens each: 2.76 ms a step
+        with the 1 split of 64 rows, 2.77 with the 2 of 32). Elsewhere another order is a rounding of bf16, and the whole step's
+        plan is the faster one (64 users, 4 dense layers of width 5120: 1.68 ms, 1.92 with that of a half)."""
+        return B // 2 if self._halves(B) and self._holds(ops.sm100.Nv4Weight) else B
 
     def _capture(self, B: int) -> _Entry:
         eng = self.eng
@@ -95,12 +107,13 @@ class DecodeGraphs:
 
         Hkv = eng.model.n_kv_l
         G = max(1, eng.model.n_head_l // Hkv)
-        splits = ops.sm100.decode_splits(B, Hkv, (G + 15) // 16, eng.cfg.ctx_size)
+        split_seqs = self._split_seqs(B)
+        splits = ops.sm100.decode_splits(split_seqs, Hkv, (G + 15) // 16, eng.cfg.ctx_size)
         e.batch = StepBatch(
             token_ids=view("token_ids"), positions=view("positions"), cu_q=view("cu_q"), ctx_lens=view("ctx_lens"),
             block_table=view("block_table").view(B, W), slots=view("slots").view(torch.int64),
             state_slots=view("state_slots"), logit_rows=None, max_q_len=1, max_ctx=eng.cfg.ctx_size,
-            write_state=True, cu_q_host=list(range(B + 1)), decode_splits=splits)
+            write_state=True, cu_q_host=list(range(B + 1)), decode_splits=splits, split_seqs=split_seqs)
         # neutral contents for warm-up and capture: every row is a padding row
         self._fill_padding(e, 0)
         e.pack_d.copy_(e.pack_h)

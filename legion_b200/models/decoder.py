@@ -60,6 +60,7 @@ class StepBatch:
     latent_parts: Optional[list] = None          # ops.sm100.latent_parts of this step
     gdn_plan: Optional[tuple] = None             # ops.sm100.gdn_chunk_plan of this step
     decode_splits: Optional[int] = None
+    split_seqs: Optional[int] = None             # sequences that latent attention plans its key splits for (None: n_seqs)
     replay: Optional[dict] = None                # verify steps: per-layer recurrent inputs kept for commit
     rope_table: Optional[torch.Tensor] = None    # [T, rot] per-token cos | sin rows (multi-section rotary positions of
     rope_rows: Optional[torch.Tensor] = None     #   image tokens); rope_rows = arange(T) indexes it like positions
@@ -694,7 +695,7 @@ class Decoder:
         L, dn, dvh = cfg.kv_lora, cfg.qk_nope_dim, cfg.v_head_dim
         scale = cfg.attn_scale or (dn + cfg.qk_rope_dim) ** -0.5
         o_lat = ops.sm100.mla_attn(q_abs, kv.k[il], b.cu_q, b.ctx_lens, b.block_table, kv.page, b.max_q_len, scale,
-                                   max_ctx=b.max_ctx or None)
+                                   max_ctx=b.max_ctx or None, split_seqs=b.split_seqs)
         if own and isinstance(w[f"{p}.mla.kv_b"], torch.Tensor) and dvh % 8 == 0 and ops.sm100.TUNE["mla_head_gemm"]:
             out = torch.empty(T, nh * dvh, dtype=q_abs.dtype, device=q_abs.device)
             w_uv = w[f"{p}.mla.kv_b"].view(nh * (dn + dvh), L)[dn:]                       # head h: rows h*(dn+dvh)..+dvh
@@ -1156,14 +1157,15 @@ class Decoder:
         max_ctx = b.max_ctx or None
         if decode and ops.sm100.latent_decode_ok(q, cache, H, m.dim, R, L, m.vdim):
             return ops.sm100.latent_decode(q, lat, gate, uk, uv, norm, cfg.rms_eps, rot, b.positions, b.slots, cache,
-                                           b.block_table, b.ctx_lens, b.cu_q, m.scale, H, m.dim, R, max_ctx)
+                                           b.block_table, b.ctx_lens, b.cu_q, m.scale, H, m.dim, R, max_ctx, b.split_seqs)
         if isinstance(b, ops.sm100.LatentPart) and ops.sm100.latent_expand_ok(q, cache, b, H, m.dim, R, m.rot.dims, L, m.vdim):
             rows = self._latent_uk.get(p)
             if rows is None:          # the key projection as stored, [heads * dim, rank]
                 rows = self._latent_uk[p] = uk.view(H, L, m.dim).transpose(1, 2).reshape(H * m.dim, L).contiguous()
             return ops.sm100.latent_prompt(q, lat, gate, rows, uv, norm, cfg.rms_eps, rot, cache, b, m.scale, H, m.dim, R)
         q_abs = ops.latent_queries(q, lat, uk, norm, cfg.rms_eps, rot, b.positions, b.slots, cache, H, m.dim, R)
-        o = ops.latent_attention(q_abs, cache, b.block_table, b.ctx_lens, b.cu_q, b.max_q_len, m.scale, L, R, max_ctx=max_ctx)
+        o = ops.latent_attention(q_abs, cache, b.block_table, b.ctx_lens, b.cu_q, b.max_q_len, m.scale, L, R, max_ctx=max_ctx,
+                                 split_seqs=b.split_seqs if decode else None)
         return ops.latent_values(o, uv, gate)
 
     def _rglru_mixer(self, p: str, il: int, h, b: StepBatch, st: StatePool):

@@ -936,13 +936,13 @@ def mla_prep(kva, norm_w, eps, w_offset, q, q_pe_off, cos_sin, positions, slots,
 
 
 def mla_attn(q_abs, cache, cu_q, ctx_lens, block_table, page, max_q_len, scale, n_splits=None, max_ctx=None, out=None,
-             rank: int = 512, rot: int = 64):
+             rank: int = 512, rot: int = 64, split_seqs: Optional[int] = None):
     """Latent attention, absorbed form: q_abs [T, heads, rank + rot], cache rows [.., rank + rot] (either with padding
-    columns behind) -> [T, heads, rank]."""
+    columns behind) -> [T, heads, rank]. ``split_seqs``: sequences that the key splits are planned for, if not those of the step."""
     C = ext()
     T, nh, _ = q_abs.shape
     if n_splits is None:
-        n_splits = mla_splits(int(ctx_lens.numel()), max_q_len, nh, max_ctx or block_table.shape[1] * page)
+        n_splits = mla_splits(split_seqs or int(ctx_lens.numel()), max_q_len, nh, max_ctx or block_table.shape[1] * page)
     ws = Workspace.get(q_abs.device)
     o_part = ml_part = None
     if n_splits > 1:
@@ -989,7 +989,7 @@ def latent_decode_ok(q, cache, heads: int, dim: int, rot: int, rank: int, vdim: 
 
 
 def latent_decode(q, kv, gate, uk, uv, norm_w, eps, cos_sin, positions, slots, cache, block_table, ctx_lens, cu_q, scale,
-                  heads: int, dim: int, rot: int, max_ctx=None):
+                  heads: int, dim: int, rot: int, max_ctx=None, split_seqs: Optional[int] = None):
     """One token per sequence: queries into the latent space with the cache append | attention over the latents in key
     splits | merge, value projection and output gate. [T, heads * vdim]."""
     C = ext()
@@ -998,7 +998,7 @@ def latent_decode(q, kv, gate, uk, uv, norm_w, eps, cos_sin, positions, slots, c
     bf = dict(dtype=torch.bfloat16, device=q.device)
     q_abs = torch.empty(T, heads, latent_row(L, rot), **bf)
     C.latent_prep(q, kv, norm_w, eps, cos_sin, positions, slots, cache, q_abs, dim, rot, uk, False)
-    n = mla_splits(int(ctx_lens.numel()), 1, heads, max_ctx or block_table.shape[1] * page)
+    n = mla_splits(split_seqs or int(ctx_lens.numel()), 1, heads, max_ctx or block_table.shape[1] * page)
     o_part = ml_part = o_lat = None
     if n > 1:
         o_part = ws.buf("mla_o", (T * heads * n * L,), torch.float32)
@@ -1125,11 +1125,12 @@ def mla_prompt(q, kv_b, cache, p: LatentPart, scale, heads: int, dim: int, rot: 
                         scale).view(T, heads * V)
 
 
-def latent_attention(q_abs, cache, block_table, ctx_lens, cu_q, max_q_len, scale, rank: int, rot: int, max_ctx=None):
+def latent_attention(q_abs, cache, block_table, ctx_lens, cu_q, max_q_len, scale, rank: int, rot: int, max_ctx=None,
+                     split_seqs: Optional[int] = None):
     """Causal attention over cached latent rows, [T, heads, rank]: tcgen05 in bf16, FMA units for fp32 and other sizes."""
     if latent_tc_ok(q_abs, cache, rank, rot):
         return mla_attn(q_abs, cache, cu_q, ctx_lens, block_table, cache.shape[1], max_q_len, scale, max_ctx=max_ctx, rank=rank,
-                        rot=rot)
+                        rot=rot, split_seqs=split_seqs)
     out = torch.empty(q_abs.shape[0], q_abs.shape[1], rank, dtype=q_abs.dtype, device=q_abs.device)
     ext().latent_attn_general(q_abs, cache, cu_q, ctx_lens, block_table, scale, rank, rot, out)
     return out
