@@ -145,7 +145,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int pos0 = ctx - q_len + tile_row0;                                   // absolute position of the tile's row 0
   const int rows_here = max(0, min(128, q_len - tile_row0));
   const int kv_hi = min(ctx, ctx - q_len + min(q_len, pair_row0 + 256));      // keys that the pair's last row sees
-  const int n_blk = (kv_hi + BKV - 1) / BKV;
+  const int n_blk = kv_hi > 0 ? (kv_hi + BKV - 1) / BKV : 0;                  // 0: a context shorter than the rows behind this tile
   const int* bt = a.block_table + long(seq) * a.table_width;
 
   if (warp == 0 || warp == 10) {
@@ -225,7 +225,7 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         return true;
       };
       bool ok = mbar_wait(q_full, 0, abort_flag) || fail(ST_TIMEOUT_FULL);
-      ok = ok && issue_s(0);
+      if (n_blk > 0) ok = ok && issue_s(0);
       for (int i = 0; ok && i < n_blk; ++i) {
         // buffer (i + 1) & 1 held P(i - 1), whose products have been issued: they run in order
         if (i + 1 < n_blk && !issue_s(i + 1)) break;
@@ -387,8 +387,13 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll 1
       for (int c = 0; c < OC; c += 32) {
         uint32_t o[32];
-        tmem_ld32(my_O + c, o);
-        tmem_ld_wait();
+        if (n_blk > 0) {
+          tmem_ld32(my_O + c, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j] = 0;
+        }
         if (row < rows_here) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {

@@ -143,6 +143,30 @@ def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
         assert (out[a:b].double() - want).abs().max() < 2.0 ** -6 * want.abs().max()
 
 
+# contexts shorter than their portions (and none at all): rows in front of the first token see nothing and give zeros
+@pytest.mark.parametrize("dk,dv,q_lens", [(192, 128, (700, 300, 400)), (128, 128, (2048, 300, 1100))])
+def test_prefill_attention_rows_without_a_key(dk, dv, q_lens):
+    Hq, Hkv, page, ctx = 4, 2, 64, (q_lens[0], 0, 150)
+    width, T = -(-q_lens[0] // page), sum(q_lens)
+    k, v = _rnd(3 * width, page, Hkv, dk, seed=1), _rnd(3 * width, page, Hkv, dv, seed=2)
+    q = _rnd(T, Hq, dk, seed=3)
+    bt = torch.arange(3 * width, dtype=torch.int32, device=DEV).view(3, width)
+    cu = torch.tensor([sum(q_lens[:i]) for i in range(4)], dtype=torch.int32, device=DEV)
+    out = torch.full((T, Hq, dv), 7.0, dtype=torch.bfloat16, device=DEV)
+    sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5, out=out)
+    assert sm().Workspace.get(DEV).check() == 0
+    parts = out.double().split(q_lens)
+    assert not parts[1].any() and not parts[2][:q_lens[2] - 150].any()
+    for i, n in ((0, q_lens[0]), (2, 150)):
+        kk = k[bt[i].long()].reshape(-1, Hkv, dk)[:n].double().repeat_interleave(Hq // Hkv, 1)
+        vv = v[bt[i].long()].reshape(-1, Hkv, dv)[:n].double().repeat_interleave(Hq // Hkv, 1)
+        s = torch.einsum("qhd,khd->hqk", q.split(q_lens)[i][-n:].double(), kk) * dk ** -0.5
+        s.masked_fill_(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+        want = torch.einsum("hqk,khd->qhd", s.softmax(-1), vv)
+        # bf16 probabilities and output, 2^-9 each
+        assert (parts[i][-n:] - want).norm() < 2.0 ** -8 * want.norm()
+
+
 # query and key preparation and the gate (eight columns per thread, one where rows do not lie on 16 bytes): partial and whole rotation,
 # a token without a cell, a last warp that is not full
 @pytest.mark.parametrize("T,Hq,Hkv,D,rot,gated,shift", [(5, 3, 1, 64, 64, False, 0), (130, 4, 2, 128, 128, False, 0), (33, 2, 1, 256, 64, True, 0),
