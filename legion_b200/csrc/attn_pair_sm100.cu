@@ -17,6 +17,7 @@
 // the barriers without touching tensor memory, so that nobody is left behind.
 #include "cluster_pair.cuh"
 #include "kernels.h"
+#include "pair_launch.h"
 #include "tmap.cuh"
 
 namespace lb {
@@ -442,7 +443,6 @@ int start(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, c
 
 }  // namespace
 
-// tq, tk, tv: the maps of attn_prefill_sm100.cu (boxes of 64 columns, 128 query rows or one page). -1: not for these sizes.
 int pair_attn_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const int* cu_q, const int* ctx_lens,
                      const int* block_table, int table_width, int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk,
                      int dv, float scale_log2, void* out, int* status, cudaStream_t s) {

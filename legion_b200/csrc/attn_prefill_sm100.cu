@@ -24,6 +24,7 @@
 #include "attn_extra.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "pair_launch.h"
 #include "tmap.cuh"
 
 namespace lb {
@@ -522,10 +523,6 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
 }
 
-int pair_attn_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const int* cu_q, const int* ctx_lens,
-                     const int* block_table, int table_width, int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk,
-                     int dv, float scale_log2, void* out, int* status, cudaStream_t s);
-
 namespace {
 thread_local char g_attn_err[256];
 
@@ -560,7 +557,7 @@ const char* prefill_attn_last_error() { return g_attn_err; }
 int prefill_attn_launch(const void* q, long T, const void* k_cache, const void* v_cache, long n_cells, long k_cell,
                         long v_cell, const int* cu_q, const int* ctx_lens, const int* block_table, int table_width,
                         int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk, int dv, float scale, float softcap,
-                        int window, int causal, void* out, int* status, cudaStream_t s, const AttnExtra& x) {
+                        int window, int causal, void* out, int* status, cudaStream_t s, int pairs, const AttnExtra& x) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
   const int DK = dk <= 64 ? 64 : (dk <= 128 ? 128 : 256), DV = dv <= 64 ? 64 : (dv <= 128 ? 128 : (dv <= 192 ? 192 : 256));
   const bool cap = softcap > 0.f;
@@ -598,10 +595,8 @@ int prefill_attn_launch(const void* q, long T, const void* k_cache, const void* 
     a.scale_log2 = 2.f * 1.4426950408889634f * softcap;
   }
   a.out = static_cast<__nv_bfloat16*>(out); a.dk = dk; a.dv = dv; a.status = status;
-  // plain causal prompts of more than one tile of rows: pairs of SMs share keys and values (attn_pair_sm100.cu)
-  // (at head sizes to 128 two single CTAs fit an SM and hide one another's waits: 32 heads, 9 x 600 tokens 113 us against 144,
-  // 4 x 1200 144 against 140, 2048 93 against 77)
-  if (!x.on && !cap && window == 0 && causal && max_q_len > (dk <= 128 ? 1023 : 128)) {
+  // plain causal prompts: pairs of SMs share keys and values (attn_pair_sm100.cu) where the caller's rule says so
+  if (pairs && !x.on && !cap && window == 0 && causal) {
     const int rc = pair_attn_launch(tq, tk, tv, cu_q, ctx_lens, block_table, table_width, page, n_seqs, max_q_len, Hq, Hkv, dk, dv,
                                     a.scale_log2, out, status, s);
     if (rc > 0) snprintf(g_attn_err, sizeof(g_attn_err), "prefill attention: launch on pairs: %s", cudaGetErrorString(cudaGetLastError()));

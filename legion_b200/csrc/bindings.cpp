@@ -430,13 +430,13 @@ void prefill_attn_ext(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
                                          long(Hkv) * D, long(Hkv) * DV, cu_q.data_ptr<int>(), ctx_lens.data_ptr<int>(),
                                          block_table.data_ptr<int>(), int(block_table.size(1)), page, int(ctx_lens.numel()),
                                          int(max_q_len), Hq, Hkv, D, DV, float(scale), 0.f, int(window), 1, out.data_ptr(),
-                                         reinterpret_cast<int*>(status.data_ptr()), cur_stream(), x);
+                                         reinterpret_cast<int*>(status.data_ptr()), cur_stream(), 0, x);
   TORCH_CHECK(rc == 0, lb::prefill_attn_last_error());
 }
 
 void prefill_attn(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& cu_q,
                   const Tensor& ctx_lens, const Tensor& block_table, int64_t max_q_len, double scale, int64_t window,
-                  bool causal, Tensor& out, Tensor& status, double softcap) {
+                  bool causal, Tensor& out, Tensor& status, double softcap, bool pairs) {
   check_bf16(q, "q");
   TORCH_CHECK(q.is_contiguous() && out.is_contiguous(), "prefill_attn: q/out must be contiguous [T, Hq, D]");
   c10::cuda::CUDAGuard guard(q.device());
@@ -452,7 +452,7 @@ void prefill_attn(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache,
                                          int(ctx_lens.numel()), int(max_q_len), Hq, Hkv, D, DV, float(scale),
                                          float(softcap), int(window),
                                          causal ? 1 : 0, out.data_ptr(), reinterpret_cast<int*>(status.data_ptr()),
-                                         cur_stream());
+                                         cur_stream(), pairs ? 1 : 0);
   TORCH_CHECK(rc == 0, lb::prefill_attn_last_error());
 }
 

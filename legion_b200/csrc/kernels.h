@@ -42,7 +42,8 @@ const char* paged_decode_tc_last_error();
 int prefill_attn_launch(const void* q, long T, const void* k_cache, const void* v_cache, long n_cells, long k_cell,
                         long v_cell, const int* cu_q, const int* ctx_lens, const int* block_table, int table_width,
                         int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk, int dv, float scale, float softcap,
-                        int window, int causal, void* out, int* status, cudaStream_t s, const AttnExtra& x = AttnExtra{});
+                        int window, int causal, void* out, int* status, cudaStream_t s, int pairs,
+                        const AttnExtra& x = AttnExtra{});
 const char* prefill_attn_last_error();
 
 // Latent attention (absorbed form) over the paged latent cache: attn_mla_sm100.cu

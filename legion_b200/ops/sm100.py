@@ -809,14 +809,53 @@ def paged_decode(q, k_cache, v_cache, block_table, ctx_lens, scale, window=0, n_
     return out
 
 
+# Prompt attention in us, as fitted to the times below (10% off at most sizes): the key-steps of all tiles over the SMs or the
+# last tile's chain, whichever is longer, and a share of the other. Per head class and kernel: rows of a tile, tiles that run
+# side by side, fixed time, time of a tile, per key of a tile, per key of a tile that runs alone, share.
+_ATTN_TIME = {
+    (False, False): (128, 296, 1.0, 8.9, 0.0269, 0.0196, 0.56), (False, True): (256, 74, 3.2, 7.8, 0.0106, 0.0069, 0.66),
+    (True, False): (128, 148, 6.0, 5.5, 0.0277, 0.0214, 0.45), (True, True): (256, 74, 8.5, 7.2, 0.0119, 0.0084, 0.28),
+}
+
+
+@functools.lru_cache(maxsize=4096)
+def attn_on_pairs(T: int, n_seqs: int, max_q_len: int, ctx: int, heads: int, dk: int) -> bool:
+    """Whether plain causal attention over ``T`` query rows of ``n_seqs`` sequences, the longest ``max_q_len`` behind a context of
+    ``ctx`` keys, runs on pairs of SMs (``attn_pair_sm100.cu``): where the modelled time of the longest sequence beside others
+    of equal length is 5% below that of single CTAs. A pair takes 256 rows at a time: it loses where short sequences fill its
+    tiles badly, and at head sizes to 128, where two single CTAs share an SM, up to about 1000 rows.
+    Single CTAs / pairs, us. 32 heads of 128 over 4 key heads: 1100 rows 48 / 50, beside 15 sequences of 80 rows 60 / 107, beside
+    8 of 300 78 / 121; 2048 97 / 85, beside 15 of 128 109 / 154, behind 2048 keys 199 / 158; 4096 263 / 230. 32 heads of 192 (values
+    128): 256 rows 18 / 22, 384 21 / 19, 1024 60 / 37, 130 behind 2048 keys 76 / 41, 1100 beside 15 of 80 97 / 113, 2048 beside 15
+    of 128 185 / 164, 4096 486 / 232."""
+    wide = dk > 128
+    if max_q_len <= (128 if wide else 1023) or ctx < 384:
+        return False
+    behind = max(0, ctx - max_q_len)
+    rest = max(0, T - max_q_len) // (n_seqs - 1) if n_seqs > 1 else 0
+
+    def time(rows, slots, fixed, tile, key, alone, share):
+        n, keys = 0, 0.0
+        for length, count in ((max_q_len, 1), (rest, n_seqs - 1)):
+            t = count * -(-length // rows)
+            n, keys = n + t, keys + t * (behind + (length + rows) / 2)
+        work, chain = heads * (n * tile + keys * key) / slots, tile + (behind + max_q_len) * alone
+        return fixed + max(work, chain) + share * min(work, chain)
+    return 1.05 * time(*_ATTN_TIME[wide, True]) < time(*_ATTN_TIME[wide, False])
+
+
 def prefill_attn(q, k_cache, v_cache, cu_q, ctx_lens, block_table, max_q_len, scale, window=0, causal=True, out=None,
-                 softcap=0.0):
+                 softcap=0.0, pairs: Optional[bool] = None):
+    """``pairs``: on pairs of SMs or on single CTAs (None: ``attn_on_pairs``)."""
     C = ext()
+    if pairs is None:
+        pairs = attn_on_pairs(q.shape[0], ctx_lens.shape[0], max_q_len, block_table.shape[1] * k_cache.shape[1], q.shape[1],
+                              q.shape[2])
     if out is None:
         out = torch.empty(q.shape[0], q.shape[1], v_cache.shape[3], dtype=q.dtype, device=q.device)
     ws = Workspace.get(q.device)
     C.prefill_attn(q, k_cache, v_cache, cu_q, ctx_lens, block_table, max_q_len, scale, window, causal, out, ws.status,
-                   float(softcap))
+                   float(softcap), pairs)
     return out
 
 
