@@ -61,13 +61,22 @@ class DecodeGraphs:
         return off, o
 
     def _lanes(self, B: int) -> int:
-        """Concurrent lanes of a decode step: one. On request (``decode_lanes`` 2) the batch runs from 64 rows on as two
-        independent halves on parallel branches of the graph, which fill each other's gaps but read every weight twice. One
-        lane wins since its kernels have variants for 64 rows: 64 users, 8 layers of the 80B-A3B shape 2.94 against 3.20 ms, 4 of
-        the 30B-A3B 1.69 / 1.80, 4 dense layers of width 5120 1.43 / 1.56, 6 of latent attention 1.36 / 1.48. Never two
-        for ranks that take part in collectives (their order must be the same on every rank), for offloaded experts, and
-        for models whose sublayers run on branches of their own (``Decoder._branch``)."""
-        return 2 if self._halves(B) and int(ops.sm100.TUNE.get("decode_lanes", 1)) >= 2 else 1
+        """Concurrent lanes of a decode step. With two (always from 64 rows on if ``decode_lanes`` is 2) the halves run on parallel
+        branches of the graph, which fill each other's gaps but read every weight twice. One lane wins where its kernels have
+        variants for the whole: 64 users, 8 layers of the 80B-A3B shape 2.65 against 2.84 ms, 4 of the 30B-A3B 1.69 / 2.11, 4
+        dense layers of width 5120 1.43 / 2.07, 6 of latent attention 1.32 / 2.18. Two win where the tables of decode-sized
+        routing, which end at 64 rows, still hold the halves: NVFP4 experts of 65 to 128 rows (8 layers of the 80B-A3B shape,
+        one / two lanes: 96 users 6.90 / 3.84 ms, 128 5.70 / 4.50, 192 6.87 / 12.1; 30B-A3B 96 2.17 / 1.60, 128 2.74 / 1.88), and
+        for FP8 experts, which have no sparse columns, of 64 (30B-A3B 2.20 / 1.99, 80B-A3B 4.99 / 3.94; 96 users 1.68 / 3.40,
+        4.24 / 7.31). Never two for ranks that take part in collectives (their order must be the same on every rank), for
+        offloaded experts, and for models whose sublayers run on branches of their own (``Decoder._branch``)."""
+        if not self._halves(B):
+            return 1
+        if int(ops.sm100.TUNE.get("decode_lanes", 1)) >= 2:
+            return 2
+        experts = [t for k, t in self.eng.model.w.items() if ".moe." in k]
+        four, eight = (any(isinstance(t, kind) for t in experts) for kind in (ops.sm100.Nv4Weight, ops.sm100.Fp8Weight))
+        return 2 if (four and 64 < B <= 128) or (eight and B == 64) else 1
 
     def _halves(self, B: int) -> bool:
         """Whether a step of ``B`` rows may run as two halves."""

@@ -1,6 +1,9 @@
 """Rules that choose between kernels, at sizes where both sides were measured."""
+from types import SimpleNamespace
+
 import pytest
 
+from legion_b200.engine.cuda_graphs import DecodeGraphs
 from legion_b200.ops import sm100
 
 
@@ -23,3 +26,21 @@ def test_prompt_attention_takes_the_faster_kernel(longest, others, rows, cached,
 def test_prompt_attention_rule_takes_any_sizes(T, n, longest, ctx):
     for dk in (64, 128, 192, 256):
         assert isinstance(sm100.attn_on_pairs(T, n, longest, ctx, 32, dk), bool)
+
+
+# weights of the experts -> rows of a decode step that run as two halves
+@pytest.mark.parametrize("kind,two", [(None, ()), ("QWeight", ()), ("Nv4Weight", (96, 128)), ("Fp8Weight", (64,))])
+def test_decode_steps_that_run_as_two_halves(kind, two, monkeypatch):
+    monkeypatch.setitem(sm100.TUNE, "decode_lanes", 1)
+    w = {"l0.attn.o": object.__new__(sm100.Nv4Weight), "l0.mlp.down": object.__new__(sm100.Fp8Weight),
+         "l1.moe.down": object.__new__(getattr(sm100, kind)) if kind else None}
+    eng = SimpleNamespace(mcfg=SimpleNamespace(parallel_sublayers=False), dp_world=1,
+                          model=SimpleNamespace(w=w, pctx=SimpleNamespace(world=1), expert_cache=None))
+    g = SimpleNamespace(eng=eng)
+    g._halves = lambda B: DecodeGraphs._halves(g, B)
+    rows = (1, 48, 64, 96, 128, 192, 256)
+    assert tuple(B for B in rows if DecodeGraphs._lanes(g, B) == 2) == two
+    monkeypatch.setitem(sm100.TUNE, "decode_lanes", 2)
+    assert tuple(B for B in rows if DecodeGraphs._lanes(g, B) == 2) == (64, 96, 128, 192, 256)
+    eng.model.pctx.world = 2
+    assert all(DecodeGraphs._lanes(g, B) == 1 for B in rows)
