@@ -43,7 +43,8 @@ void wgemm(const Tensor& w, const Tensor& x, Tensor& out, const OptT& residual, 
            const OptT& ws, const OptT& counters, Tensor& status, const OptT& tile_group, const OptT& tile_tok0,
            const OptT& tile_ntok, const OptT& meta, int64_t max_tiles, int64_t rows_per_group, int64_t n_tok,
            std::vector<int64_t> out_peer, const OptT& tile_out0, const OptT& w_scales, const OptT& w_gscale,
-           int64_t x_group_col, int64_t k_override, int64_t act, const OptT& xielu, bool relu2, const OptT& bias) {
+           int64_t x_group_col, int64_t k_override, int64_t act, const OptT& xielu, bool relu2, const OptT& bias,
+           int64_t n_groups) {
   const bool fp4 = w_scales.has_value();     // w = NVFP4 codes [rows, K/2] uint8, w_scales = e4m3 bytes [rows, K/16]
   if (fp4) {
     TORCH_CHECK(w.scalar_type() == at::kByte && w_scales->is_contiguous() && w_scales->element_size() == 1 &&
@@ -94,6 +95,9 @@ void wgemm(const Tensor& w, const Tensor& x, Tensor& out, const OptT& residual, 
   h.n_tiles_dev = optp<int>(meta);
   h.tile_out0 = optp<int>(tile_out0);
   h.n_tok_tiles_max = int(max_tiles);
+  TORCH_CHECK(n_groups == 0 || (n_groups > 0 && n_tok <= x.size(0) && out.size(0) >= n_groups * n_tok &&
+                                x_group_col * (n_groups - 1) + h.K <= x.size(1)), "wgemm: groups over all tokens: shapes");
+  h.n_groups = int(n_groups);
   h.rows_per_group = int(rows_per_group); h.dual_offset = int(dual_offset);
   h.split_k = int(split_k);
   h.ws = optpm<float>(ws);
@@ -683,7 +687,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("n_tok"), pybind11::arg("out_peer"), pybind11::arg("tile_out0") = pybind11::none(),
         pybind11::arg("w_scales") = pybind11::none(), pybind11::arg("w_gscale") = pybind11::none(),
         pybind11::arg("x_group_col") = 0, pybind11::arg("k_override") = 0, pybind11::arg("act") = 0,
-        pybind11::arg("xielu") = pybind11::none(), pybind11::arg("relu2") = false, pybind11::arg("bias") = pybind11::none());
+        pybind11::arg("xielu") = pybind11::none(), pybind11::arg("relu2") = false, pybind11::arg("bias") = pybind11::none(),
+        pybind11::arg("n_groups") = 0);
   m.def("wgemm_fp8", &wgemm_fp8);
   m.def("wgemm_fp8_q", &wgemm_fp8_q);
   m.def("wgemm_allreduce", &wgemm_allreduce);

@@ -305,7 +305,7 @@ int start(const WgemmHost& h, const WgemmArgs& a, int grid, cudaStream_t stream,
 
 bool wgemm_pair_ok(const WgemmHost& h, const WgemmArgs& a, int sms) {
   if (h.out_f32 || h.w_scales || h.w_bscale || h.xielu || h.relu2 || h.bias || h.comm.enabled || h.head.enabled ||
-      h.n_out_peer > 0 || h.x_group_col != 0 || a.split_k > 1 || !a.vec_ok || h.K < 512)
+      h.n_out_peer > 0 || h.x_group_col != 0 || h.n_groups > 0 || a.split_k > 1 || !a.vec_ok || h.K < 512)
     return false;
   // grouped tiles of 128 tokens are bound by what L2 delivers, 48 KB per k block and pair or CTA. 128 experts of 2048 x 768,
   // 44,000 token rows: down projection 222 us on pairs, 317 us by single CTAs; gate and up 372 and 291

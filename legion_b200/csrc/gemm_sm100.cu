@@ -94,6 +94,12 @@ __device__ __forceinline__ bool decode_work(const WgemmArgs& a, int w, int n_tok
     it.tok0 = a.tile_tok0[tt];
     it.out0 = a.tile_out0 ? a.tile_out0[tt] : it.tok0;
     it.ntok = a.tile_ntok[tt];
+  } else if (a.n_groups > 0) {
+    const int per_group = (a.n_tok + BN - 1) / BN;
+    it.group = tt / per_group;
+    it.tok0 = (tt - it.group * per_group) * BN;
+    it.out0 = it.tok0 * a.n_groups + it.group;
+    it.ntok = min(BN, a.n_tok - it.tok0);
   } else {
     it.group = 0;
     it.tok0 = tt * BN;
@@ -101,6 +107,12 @@ __device__ __forceinline__ bool decode_work(const WgemmArgs& a, int w, int n_tok
     it.ntok = min(BN, a.n_tok - it.tok0);
   }
   return true;
+}
+
+// output row of token t of the tile (negative = drop)
+__device__ __forceinline__ long out_row(const WgemmArgs& a, const WorkItem& it, int t) {
+  if (a.out_rows) return long(a.out_rows[it.out0 + t]);
+  return it.out0 + t * (a.n_groups > 0 ? a.n_groups : 1);
 }
 
 // four e4m3 (fn) bytes -> f16 pairs (hardware conversion; every e4m3 value is exact in f16), NaN patterns as 0
@@ -268,7 +280,7 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     asm volatile("fence.proxy.async;" ::: "memory");   // generic-proxy stores above -> TMA reads below
   }
 
-  const int n_tok_tiles = a.tile_group ? min(*a.n_tiles_dev, a.n_tok_tiles_max) : (a.n_tok + BN - 1) / BN;
+  const int n_tok_tiles = a.tile_group ? min(*a.n_tiles_dev, a.n_tok_tiles_max) : (a.n_tok + BN - 1) / BN * max(1, a.n_groups);
   const int num_kb = (a.K + KBE - 1) / KBE;
   const int kb_per_split = (num_kb + a.split_k - 1) / a.split_k;
 
@@ -727,7 +739,7 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 #pragma unroll
               for (int pass = 0; pass < 4; ++pass) {
                 const int t = c + pass * 8 + (etid >> 4);
-                orows[pass] = t < it.ntok ? (a.out_rows ? long(a.out_rows[it.out0 + t]) : long(it.out0 + t)) : -1;
+                orows[pass] = t < it.ntok ? out_row(a, it, t) : -1;
               }
             }
 #pragma unroll
@@ -782,9 +794,9 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
               const int t = c + j;
               if (t < it.ntok && feat8 < a.n_feat) {
                 const int xrow = it.out0 + t;
-                long orow = xrow;
+                long orow;
                 if constexpr (BN > 32) orow = orows[pass];
-                else if (a.out_rows) orow = a.out_rows[xrow];
+                else orow = out_row(a, it, t);
                 if (orow >= 0) {
                   __nv_bfloat16* obase = reinterpret_cast<__nv_bfloat16*>(a.out);
                   if (a.n_out_peer > 0) {
@@ -824,7 +836,7 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 #pragma unroll
             for (int pass = 0; pass < 8; ++pass) {
               const int t = c + pass * 4 + (etid >> 5);
-              orows[pass] = t < it.ntok ? (a.out_rows ? long(a.out_rows[it.out0 + t]) : long(it.out0 + t)) : -1;
+              orows[pass] = t < it.ntok ? out_row(a, it, t) : -1;
             }
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -862,8 +874,7 @@ wgemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                 float v = g[j];
                 if (DUAL) v = gate_act(v, a.act) * u[j];
                 if (a.tok_scale) v *= a.tok_scale[xrow];
-                long orow = xrow;
-                if (a.out_rows) orow = a.out_rows[xrow];
+                long orow = out_row(a, it, t);
                 if (orow >= 0) {
                   void* obase = a.out;
                   if (a.n_out_peer > 0) {
@@ -1063,11 +1074,18 @@ int wgemm_launch(const WgemmHost& h, cudaStream_t stream) {
   a.rows_per_group = h.rows_per_group; a.dual_offset = h.dual_offset; a.act = h.act; a.numbers = h.bias ? h.bias : h.xielu;
   a.x_group_col = h.x_group_col;
   // (a last K tile that reaches into the next group's columns meets weights that TMA filled with zeros)
-  if (h.x_group_col != 0 && (h.x_group_col % 8 != 0 || h.K % 8 != 0 || fp8 || fp4 || !h.tile_group)) {
+  if (h.x_group_col != 0 && (h.x_group_col % 8 != 0 || h.K % 8 != 0 || fp8 || fp4 || (!h.tile_group && h.n_groups <= 0))) {
     snprintf(g_gemm_err, sizeof(g_gemm_err),
              "wgemm: per-group activation columns need grouped bf16 mode, K %% 8 == 0 and 16-byte aligned offsets");
     return 1;
   }
+  if (h.n_groups != 0 && (h.n_groups < 0 || h.tile_group || h.out_rows || h.tok_scale || h.residual || h.dual || fp8 || fp4 || h.split_k > 1 ||
+                          h.comm.enabled || h.head.enabled || h.n_out_peer > 0 || long(h.n_groups) * h.n_tok > INT_MAX ||
+                          h.w_rows < long(h.n_groups - 1) * h.rows_per_group + h.n_feat)) {
+    snprintf(g_gemm_err, sizeof(g_gemm_err), "wgemm: groups over all tokens come with plain bf16 weights of every group and plain rows");
+    return 1;
+  }
+  a.n_groups = h.n_groups;
   a.split_k = h.split_k < 1 ? 1 : h.split_k;
   a.ws = h.ws; a.counters = h.counters; a.status = h.status;
   a.n_out_peer = h.n_out_peer;
@@ -1094,7 +1112,7 @@ int wgemm_launch(const WgemmHost& h, cudaStream_t stream) {
     snprintf(g_gemm_err, sizeof(g_gemm_err), "wgemm: split-K needs a workspace and counters");
     return 1;
   }
-  const int n_tok_tiles = h.tile_group ? h.n_tok_tiles_max : (h.n_tok + bn - 1) / bn;
+  const int n_tok_tiles = h.tile_group ? h.n_tok_tiles_max : (h.n_tok + bn - 1) / bn * (h.n_groups > 0 ? h.n_groups : 1);
   long total = long(n_tok_tiles) * a.feat_tiles * a.split_k;
   if (total <= 0) return 0;
   int grid = int(total < g_num_sms ? total : g_num_sms);

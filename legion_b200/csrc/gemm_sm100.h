@@ -56,6 +56,8 @@ struct WgemmArgs {
   const int* tile_ntok;           //   valid rows in the tile
   const int* n_tiles_dev;         //   number of token tiles (device scalar, data of a CUDA graph)
   int n_tok_tiles_max;
+  int n_groups;                   // > 0: every group multiplies all n_tok tokens (no tile list); token t of group g becomes
+                                  //   output row t * n_groups + g
   int rows_per_group;             // weight rows between consecutive groups
   int x_group_col;                // grouped mode: first activation column of group g is g * x_group_col (per-head
                                   //   projections read their head's slice of a [tokens, heads * width] tensor in place)
@@ -95,6 +97,7 @@ struct WgemmHost {
   const int* tile_group; const int* tile_tok0; const int* tile_ntok; const int* n_tiles_dev;
   const int* tile_out0;
   int n_tok_tiles_max;
+  int n_groups;                   // see WgemmArgs::n_groups
   int rows_per_group, dual_offset;
   int x_group_col; long x_cols;   // see WgemmArgs::x_group_col; x_cols: columns of the activation tensor (0 = K)
   int split_k; float* ws; int* counters;

@@ -922,34 +922,17 @@ def head_linear(x, w2d, n_heads: int, rows_per_group: int, n_feat: int, K: int, 
     ``out2d[t * n_heads + h, :n_feat] = W_h @ x[t, h * x_group_col : h * x_group_col + K]`` (0: every head reads the
     same K columns) with
     ``W_h = w2d[h * rows_per_group : h * rows_per_group + n_feat]``. One grouped launch of the tcgen05 GEMM (group =
-    head); the activation tile of a head is fetched from its column slice of ``x`` by the TMA load, the output rows
-    go through a row map, so nothing is transposed or copied."""
+    head); the activation tile of a head is fetched from its column slice of ``x`` by the TMA load and the kernel
+    computes the output rows, so nothing is transposed or copied and no tables are kept for the token counts seen."""
     C = ext()
     T = x.shape[0]
     if not (tma_ok(x, w2d) and x_group_col % 8 == 0):
         # fp32 and unaligned shapes: the FMA kernel
         C.sgemm_heads(w2d, x, out2d.view(T, -1), n_heads, rows_per_group, n_feat, K, x_group_col, out2d.shape[1])
         return out2d
-    ws = Workspace.get(x.device)
-    bn = pick_bn(T, False)
-    key = ("head_linear", T, n_heads, bn)
-    tab = ws._cache.get(key)
-    if tab is None:
-        n_tt = (T + bn - 1) // bn
-        Tp = n_tt * bn
-        h = torch.arange(n_heads).repeat_interleave(n_tt)
-        tt = torch.arange(n_tt).repeat(n_heads)
-        rows = torch.full((n_heads, Tp), -1, dtype=torch.int32)
-        rows[:, :T] = torch.arange(T) * n_heads + torch.arange(n_heads)[:, None]
-        rows = rows.view(-1)
-        i32 = dict(dtype=torch.int32, device=x.device)
-        tab = (h.to(**i32), (tt * bn).to(**i32), torch.clamp(T - tt * bn, max=bn).to(**i32),
-               (h * Tp + tt * bn).to(**i32), rows.to(x.device),
-               torch.tensor([n_heads * n_tt, 0], **i32), n_heads * n_tt)
-        ws._cache[key] = tab
-    tile_group, tile_tok0, tile_ntok, tile_out0, out_rows, meta, n_tiles = tab
-    C.wgemm(w2d, x, out2d, None, None, out_rows, n_feat, False, 0, bn, 1, None, None, ws.status, tile_group, tile_tok0,
-            tile_ntok, meta, n_tiles, rows_per_group, 0, [], tile_out0, None, None, x_group_col, K if x_group_col else 0)
+    C.wgemm(w2d, x, out2d, None, None, None, n_feat, False, 0, pick_bn(T, False), 1, None, None, Workspace.get(x.device).status,
+            None, None, None, None, 0, rows_per_group, T, [], None, None, None, x_group_col, K if x_group_col else 0,
+            n_groups=n_heads)
     return out2d
 
 

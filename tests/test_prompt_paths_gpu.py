@@ -143,6 +143,24 @@ def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
         assert (out[a:b].double() - want).abs().max() < 2.0 ** -6 * want.abs().max()
 
 
+# tiles of 32, 64, 128 and 256 tokens with a remainder, several per head; rows of an odd width leave one by one
+@pytest.mark.parametrize("T", [1, 33, 100, 257, 1000])
+@pytest.mark.parametrize("nh,nf,rows", [(3, 128, 192), (5, 72, 72), (2, 130, 256)])
+@pytest.mark.parametrize("own", [False, True])
+def test_per_head_products_keep_nothing_for_a_token_count(T, nh, nf, rows, own):
+    K = 64
+    x, w = _rnd(T, nh * K if own else K), _rnd(nh * rows, K, scale=K ** -0.5, seed=1)
+    cache = sm().Workspace.get(DEV)._cache
+    before = set(cache)
+    out = torch.full((T * nh + 4, nf), 3.0, dtype=torch.bfloat16, device=DEV)
+    sm().head_linear(x, w, nh, rows, nf, K, K if own else 0, out[:T * nh])
+    assert set(cache) == before and sm().Workspace.get(DEV).check() == 0
+    wh = w.view(nh, rows, K)[:, :nf].double()
+    want = torch.einsum("thk,hnk->thn" if own else "tk,hnk->thn", x.double().view(T, nh, K) if own else x.double(), wh)
+    assert (out[:T * nh].view(T, nh, nf).double() - want).abs().max() < 2.0 ** -8 * want.abs().max()      # one bf16 rounding
+    assert (out[T * nh:] == 3).all()
+
+
 # contexts shorter than their portions (and none at all): rows in front of the first token see nothing and give zeros
 @pytest.mark.parametrize("dk,dv,q_lens", [(192, 128, (700, 300, 400)), (128, 128, (2048, 300, 1100))])
 def test_prefill_attention_rows_without_a_key(dk, dv, q_lens):
