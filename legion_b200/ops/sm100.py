@@ -1359,6 +1359,8 @@ def _moe_experts_nv4(x, ids, wts, w_gate_up: "Nv4Weight", w_down: "Nv4Weight", n
     """Routed experts on the native NVFP4 path (decode-sized steps over the dense routing): the layer input is
     quantised once (or arrives quantised as ``xq``), the gate/up GEMM re-encodes its SwiGLU output to NVFP4 in its
     epilogue (static tensor scale ``h_scale``), and the down GEMM reads that. Three launches + the combine."""
+    if routing.shared_rows:
+        raise NotImplementedError("always-chosen experts in the routing tables come with bf16 weights")
     C = ext()
     T, H = x.shape
     k = ids.shape[1]

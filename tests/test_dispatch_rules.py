@@ -2,6 +2,7 @@
 from types import SimpleNamespace
 
 import pytest
+import torch
 
 from legion_b200.engine.cuda_graphs import DecodeGraphs
 from legion_b200.ops import sm100
@@ -44,3 +45,14 @@ def test_decode_steps_that_run_as_two_halves(kind, two, monkeypatch):
     assert tuple(B for B in rows if DecodeGraphs._lanes(g, B) == 2) == (64, 96, 128, 192, 256)
     eng.model.pctx.world = 2
     assert all(DecodeGraphs._lanes(g, B) == 1 for B in rows)
+
+
+def test_nvfp4_experts_refuse_always_chosen_experts_in_the_tables():
+    """Their tile bound and their combine know the pairs and one shared slot."""
+    E, k, T = 8, 2, 3
+    w = sm100.Nv4Weight(torch.zeros(E + 2, 512, 128, dtype=torch.uint8), None, torch.ones(E + 2))
+    ids = torch.zeros(T, k, dtype=torch.int32)
+    r = sm100.Routing(ids, torch.ones(T, k), SimpleNamespace(n_slots=E + 2, bn=32, stride=32, hq=None, y_pairs=None), None, 0, E)
+    r.shared_rows = 2
+    with pytest.raises(NotImplementedError):
+        sm100._moe_experts_nv4(torch.zeros(T, 256, dtype=torch.bfloat16), ids, r.wts, w, w, 256, 0, None, None, None, None, None, r)
