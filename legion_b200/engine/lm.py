@@ -267,8 +267,13 @@ class LmEngine(Engine):
             del sp
         free, total = torch.cuda.mem_get_info(dev)
         m = self.mcfg
+        latent = 0
+        if "mla" in m.layer_kinds and model.dtype == torch.bfloat16:
+            from ..ops import sm100
+            latent = sm100.mla_expand_bytes(c.max_batch_tokens, c.max_seqs, c.ctx_size, model.n_head_l, m.qk_nope_dim, m.qk_rope_dim,
+                                            m.v_head_dim, m.kv_lora)
         ws = mp.workspace_reserve(m.hidden, m.vocab, c.max_batch_tokens, c.max_seqs, m.n_expert, m.top_k, m.expert_ff,
-                                  m.stream_rows())
+                                  m.stream_rows(), latent)
         auto = c.kv_cache_tokens is not None and c.kv_cache_tokens < 0
         asked = 0 if auto else n_blocks * c.block_size
         plan = mp.fit(total, free, torch.cuda.memory_allocated(dev), bpb, c.block_size, state_bytes, ws, c.max_seqs,

@@ -1130,6 +1130,13 @@ def mla_expand_ok(q, kv_b, cache, p: LatentPart, heads: int, dim: int, rot: int,
     return scratch <= max(MLA_EXPAND_FREE, q.shape[0] * heads * (2 * rank + rot) * 2)
 
 
+def mla_expand_bytes(max_tokens: int, max_seqs: int, ctx: int, heads: int, dim: int, rot: int, vdim: int, rank: int) -> int:
+    """The most scratch that ``mla_expand_ok`` grants a step of ``max_tokens`` tokens over sequences of up to ``ctx`` each."""
+    portions = min(max_seqs, max_tokens // LATENT_EXPAND_MIN)
+    cells = portions * -(-ctx // 64) * 64 * (heads * (dim + rot + vdim) + rank) * 2
+    return min(cells, max(MLA_EXPAND_FREE, max_tokens * heads * (2 * rank + rot) * 2))
+
+
 def mla_prompt(q, kv_b, cache, p: LatentPart, scale, heads: int, dim: int, rot: int, rank: int):
     """Long portions of a latent-attention layer in the per-head form (``latent_prompt``): q [T, heads, dim + rot] turned,
     kv_b [heads * (dim + vdim), rank] as stored, the tokens' cells written. [T, heads * vdim].

@@ -56,3 +56,34 @@ def test_nvfp4_experts_refuse_always_chosen_experts_in_the_tables():
     r.shared_rows = 2
     with pytest.raises(NotImplementedError):
         sm100._moe_experts_nv4(torch.zeros(T, 256, dtype=torch.bfloat16), ids, r.wts, w, w, 256, 0, None, None, None, None, None, r)
+
+
+# tokens of a step and context: the smallest long portion behind a long history, one at the limit, a whole prompt
+@pytest.mark.parametrize("tokens,ctx", [(192, 4096), (192, 65536), (2048, 16384), (4096, 4096), (300, 512)])
+def test_memory_plan_counts_the_expanded_keys_of_latent_prompts(tokens, ctx, monkeypatch):
+    from legion_b200.config import ModelConfig
+    from legion_b200.engine import memory_plan
+    from legion_b200.engine.lm import EngineConfig, LmEngine
+    heads, dim, rot, vdim, rank, seqs = 8, 128, 64, 128, 512, 3
+    kv_b, cache = torch.empty(heads * (dim + vdim), rank, dtype=torch.bfloat16), torch.empty(1, 64, 1, rank + rot, dtype=torch.bfloat16)
+    q = torch.empty(tokens, heads, dim + rot, dtype=torch.bfloat16)
+    most = 0
+    for portions in range(1, seqs + 1):
+        if tokens // portions < sm100.LATENT_EXPAND_MIN:
+            continue
+        for pages in (1, ctx // 128 * portions, -(-ctx // 64) * portions):
+            p = sm100.LatentPart()
+            p.expand, p.pages = True, torch.empty(2, max(1, pages), dtype=torch.int32)
+            if sm100.mla_expand_ok(q, kv_b, cache, p, heads, dim, rot, vdim, rank):
+                most = max(most, max(1, pages) * 64 * (heads * (dim + rot + vdim) + rank) * 2)
+    granted = sm100.mla_expand_bytes(tokens, seqs, ctx, heads, dim, rot, vdim, rank)
+    assert 0 < most <= granted
+    cfg = ModelConfig(arch="deepseek_v3", n_layer=1, hidden=1024, vocab=512, n_head=heads, n_kv_head=heads, head_dim=dim + rot, kv_lora=rank,
+                      qk_nope_dim=dim, qk_rope_dim=rot, v_head_dim=vdim, qk_norm=False, dense_ff=512)
+    eng = SimpleNamespace(mcfg=cfg, ring_len=0, hybrid=False, cfg=EngineConfig(ctx_size=ctx, max_seqs=seqs, max_batch_tokens=tokens,
+                                                                              block_size=64, kv_cache_tokens=-1))
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (100 << 30, 180 << 30))
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev: 0)
+    LmEngine._plan_memory(eng, SimpleNamespace(dtype=torch.bfloat16, n_kv_l=heads, n_head_l=heads, pctx=SimpleNamespace(tp=1)),
+                          torch.device("cpu"), 0, None, 64)
+    assert eng.memory_plan.workspace_bytes == memory_plan.workspace_reserve(1024, 512, tokens, seqs, 0, 0, 0) + granted
