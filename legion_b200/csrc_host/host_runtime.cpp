@@ -345,6 +345,7 @@ static void pack_step(py::array_t<int32_t, py::array::c_style> buf, const std::v
   auto number = [](PyObject* list, Py_ssize_t i) {
     const long v = PyLong_AsLong(PyList_GET_ITEM(list, i));
     if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
+    if (v != long(int32_t(v))) throw std::runtime_error("pack_step: a value does not fit 32 bits");
     return v;
   };
   std::copy(logit_rows.begin(), logit_rows.end(), lrows);

@@ -42,3 +42,16 @@ def test_native_step_inputs_refuse_positions_beyond_the_table():
     eng = SimpleNamespace(pool=kv_blocks.BlockPool(16, 16), device=torch.device("cpu"))
     with pytest.raises(IndexError):
         LmEngine._step_inputs(eng, [(_seq([5], 3), 10, list(range(8)))], [0])
+
+
+# a token id, a rotary position: refused by both forms
+@pytest.mark.parametrize("tokens,media", [([7, 2 ** 31], None), ([-2 ** 31 - 1], None), ([7], 1)])
+def test_step_inputs_refuse_values_beyond_32_bits(tokens, media, monkeypatch):
+    eng = SimpleNamespace(pool=kv_blocks.BlockPool(16, 16), device=torch.device("cpu"))
+    seq = _seq([5], 3, media)
+    seq.rope_pos = lambda p: p + 2 ** 31
+    with pytest.raises(RuntimeError):
+        LmEngine._step_inputs(eng, [(seq, 0, tokens)], [0])
+    monkeypatch.setattr(kv_blocks, "NATIVE", None)
+    with pytest.raises(RuntimeError):
+        LmEngine._step_inputs(eng, [(seq, 0, tokens)], [0])
