@@ -40,9 +40,10 @@ def test_decode_attention_live_splits(ctx, heads, D, splits):
     assert sm().Workspace.get(DEV).check() == 0
 
 
-# token tiles of 64: an expert with a single token, with eight, nine and all of them, tokens in one half and in both
+# token tiles of 64: an expert with a single token, with eight, nine and all of them, tokens in one half and in both; the last sizes
+# have tiles for two CTAs per SM (2 x 148 of gate and up) and eight feature tiles of the down projection
 @pytest.mark.parametrize("T", [33, 40, 64])
-@pytest.mark.parametrize("E,k,H,F", [(96, 2, 256, 256), (64, 4, 512, 512)])
+@pytest.mark.parametrize("E,k,H,F", [(96, 2, 256, 256), (64, 4, 512, 512), (96, 4, 1024, 512)])
 def test_nvfp4_experts_sparse_columns(T, E, k, H, F):
     S = sm()
     gu, dn = _rnd(E, 2 * F, H, scale=H ** -0.5), _rnd(E, H, F, scale=F ** -0.5, seed=1)
@@ -71,3 +72,8 @@ def test_nvfp4_experts_sparse_columns(T, E, k, H, F):
         want.index_add_(0, t, (torch.nn.functional.silu(a) * b) @ ddn[e].t() * r.wts[t, j, None].double())
     # activations in 4 bits with a scale per 16: a tenth of their size, summed over F of them and the experts of a token
     assert (out - want).norm() < 0.12 * want.norm()
+    # the same sums as in token tiles of 32
+    for part in (slice(0, 32), slice(32, T)):
+        h = S.router(x[part].contiguous(), w_r, k, slot_stride=128)
+        assert torch.equal(h.ids, r.ids[part]) and torch.equal(h.wts, r.wts[part])
+        assert torch.equal(S.moe_experts(x[part].contiguous(), h.ids, h.wts, qgu, qdn, F, routing=h).double(), out[part])

@@ -300,9 +300,12 @@ def test_sampled_generation_on_gpu():
 
 
 @gpu
+@pytest.mark.parametrize("lanes", [1, 2])
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
-def test_many_sequences_decode_together(models, dtype):
-    """More decoded sequences than one routing tile holds; two lanes of the captured step from 64 rows on."""
+def test_many_sequences_decode_together(models, dtype, lanes, monkeypatch):
+    """More decoded sequences than one routing tile holds, in one lane of the captured step and in two."""
+    from legion_b200.ops import sm100
+    monkeypatch.setitem(sm100.TUNE, "decode_lanes", lanes)
     cfg, w, path = models.get("mixed", dtype)
     n = 70
     seqs = {f"q{i}": nc.tokens(cfg, 9 + i % 5, 200 + i) for i in range(n)}
@@ -310,6 +313,7 @@ def test_many_sequences_decode_together(models, dtype):
     r = TraceReplay(replay_engine(path, getattr(torch, dtype), n * 64, "cuda:0", slots=n))
     first = [[(k, len(v) - 4) for k, v in seqs.items()]]
     got = nc.run_schedule(r, seqs, first + [[(k, 1) for k in seqs]] * 4)
+    assert len(r.engine._graphs.entries[96].parts) == lanes
     for k in want:
         check(got[k], want[k], dtype, k)
 

@@ -68,8 +68,9 @@ def test_latent_prompt_per_head_form(lens, cached, monkeypatch):
     assert torch.equal(ka[0], kb[0]) and (ka[1] - kb[1]).norm() < 0.01 * kb[1].norm()
 
 
-# tiles of 256 tokens with a remainder, features that end inside a pair of SMs, a last K block that is not whole
-@pytest.mark.parametrize("T,N,K", [(1300, 4104, 584), (2304, 2560, 512), (1281, 4352, 1024)])
+# tiles of 256 tokens with a remainder, features that end inside a pair of SMs (of one weight, and of gate and up: 2056), a last K
+# block that is not whole
+@pytest.mark.parametrize("T,N,K", [(1300, 4104, 584), (2304, 2560, 512), (1281, 4352, 1024), (1300, 4112, 584)])
 def test_prompt_gemm_on_pairs(T, N, K):
     x, w, res = _rnd(T, K), _rnd(N, K, scale=K ** -0.5, seed=1), _rnd(T, N, seed=2)
     scale = torch.rand(T, generator=torch.Generator().manual_seed(3)).to(DEV)
@@ -86,8 +87,8 @@ def test_prompt_gemm_on_pairs(T, N, K):
 
 # groups of 0, 1, 127, 128, 129 tokens and more over token tiles of 128, both expert products
 def test_grouped_gemm_on_pairs():
-    E, H, F = 24, 512, 640
-    counts = [0, 1, 127, 128, 129, 300] * 4
+    E, H, F = 48, 512, 640
+    counts = [0, 1, 127, 128, 129, 300] * 8
     ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])
     ids = ids[torch.randperm(len(ids), generator=torch.Generator().manual_seed(0))].to(DEV)[:, None]
     T = len(ids)
@@ -96,6 +97,8 @@ def test_grouped_gemm_on_pairs():
     wts = torch.rand(T, 1, generator=torch.Generator().manual_seed(4)).to(DEV)
     out = sm().moe_experts(x, ids, wts, gu, dn, F).double()
     assert sm().Workspace.get(DEV).check() == 0
+    # the down projection runs on pairs from 64 tiles of 128 tokens on
+    assert sm().Workspace.get(DEV)._cache["moe_plan", T, 1, E, 128, H, F].max_tiles >= 64
     want = torch.empty(T, H, dtype=torch.float64, device=DEV)
     for e in range(E):
         t = (ids[:, 0] == e).nonzero()[:, 0]
@@ -119,8 +122,9 @@ def test_short_prompt_gemm(T, N, K):
 
 # pairs of 256 query rows: one row more than a tile, an empty second tile, full pairs, short sequences beside long ones, cached
 # tokens in front; blocks of 128 keys with a remainder; head sizes between and at the kernel's, pages of a part of its tiles
-@pytest.mark.parametrize("q_lens,cached,page", [([129], 0, 64), ([256, 1, 130], 70, 16), ([257, 511], 128, 32), ([1100, 128], 333, 64)])
-@pytest.mark.parametrize("Hq,Hkv,dk,dv", [(4, 2, 128, 128), (2, 2, 192, 128), (8, 1, 256, 256), (2, 1, 136, 72), (2, 1, 232, 208)])
+@pytest.mark.parametrize("q_lens,cached,page", [([129], 0, 64), ([256, 1, 130], 70, 16), ([257, 511], 128, 32), ([1100, 128], 333, 64),
+                                                ([1024], 0, 16), ([1300, 5], 61, 32)])
+@pytest.mark.parametrize("Hq,Hkv,dk,dv", [(4, 2, 128, 128), (2, 2, 192, 128), (8, 1, 160, 96), (2, 1, 136, 72), (2, 1, 72, 72)])
 def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
     n, T = len(q_lens), sum(q_lens)
     ctx = [q + cached for q in q_lens]
@@ -129,7 +133,7 @@ def test_prefill_attention_on_pairs(q_lens, cached, page, Hq, Hkv, dk, dv):
     q = _rnd(T, Hq, dk, scale=2.0, seed=3)
     bt = torch.randperm(n * width, generator=torch.Generator().manual_seed(0)).int().view(n, width).to(DEV)
     cu = torch.tensor([sum(q_lens[:i]) for i in range(n + 1)], dtype=torch.int32, device=DEV)
-    out = sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5)
+    out = sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5, pairs=True)
     assert sm().Workspace.get(DEV).check() == 0
     for i in range(n):
         kk = k[bt[i].long()].reshape(-1, Hkv, dk)[:ctx[i]].double().repeat_interleave(Hq // Hkv, 1)
@@ -163,7 +167,8 @@ def test_per_head_products_keep_nothing_for_a_token_count(T, nh, nf, rows, own):
 
 # contexts shorter than their portions (and none at all): rows in front of the first token see nothing and give zeros
 @pytest.mark.parametrize("dk,dv,q_lens", [(192, 128, (700, 300, 400)), (128, 128, (2048, 300, 1100))])
-def test_prefill_attention_rows_without_a_key(dk, dv, q_lens):
+@pytest.mark.parametrize("pairs", [False, True])
+def test_prefill_attention_rows_without_a_key(dk, dv, q_lens, pairs):
     Hq, Hkv, page, ctx = 4, 2, 64, (q_lens[0], 0, 150)
     width, T = -(-q_lens[0] // page), sum(q_lens)
     k, v = _rnd(3 * width, page, Hkv, dk, seed=1), _rnd(3 * width, page, Hkv, dv, seed=2)
@@ -171,7 +176,7 @@ def test_prefill_attention_rows_without_a_key(dk, dv, q_lens):
     bt = torch.arange(3 * width, dtype=torch.int32, device=DEV).view(3, width)
     cu = torch.tensor([sum(q_lens[:i]) for i in range(4)], dtype=torch.int32, device=DEV)
     out = torch.full((T, Hq, dv), 7.0, dtype=torch.bfloat16, device=DEV)
-    sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5, out=out)
+    sm().prefill_attn(q, k, v, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), bt, max(q_lens), dk ** -0.5, out=out, pairs=pairs)
     assert sm().Workspace.get(DEV).check() == 0
     parts = out.double().split(q_lens)
     assert not parts[1].any() and not parts[2][:q_lens[2] - 150].any()
