@@ -473,14 +473,17 @@ def pick_bn(n_tok: int, dual: bool) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
-def _pick_tile(T: int, n_feat: int, K: int, dual: bool):
-    """(token tile, K splits) of a bf16 GEMM with more than 32 tokens that does not fill the pairs of SMs
-    (``gemm_pair_sm100.cu``). The splits are those of the widest token tile, so that the sums, and with them the 4-bit
-    activations behind them, do not depend on the tile; the tile is the one with the least modelled time, in cycles. A k block of
-    64 costs what its operands move through shared memory in and out at 128 bytes per cycle, 32 columns of accumulators about
-    1400 cycles on their way out; a split adds its partial sums. With the widest tile short prompts ran on a few SMs, whose last
-    CTAs added up to nine partial sums of 256 tokens each."""
-    ft, nw, num_kb = (n_feat + 127) // 128, 2 if dual else 1, (K + 63) // 64
+def _pick_tile(T: int, n_feat: int, K: int, dual: bool, f32: bool = False):
+    """(token tile, K splits) of a bf16 GEMM with more than 32 tokens. The splits are those of the widest token tile, so that the sums,
+    and with them the 4-bit activations behind them, do not depend on the tile. With the widest tile short prompts ran on
+    a few SMs, whose last CTAs added up to nine partial sums of 256 tokens each: the tile is the narrowest with which all work
+    items still run at once, else the widest (more items than SMs repeat the weights' way through shared memory and the
+    partial sums' way through memory). float32 rows leave 32-token tiles one element at a time: 64 at least.
+    Widest / this, us: 512 x 2048, 128 tokens 26.6 / 14.4 (128 items of 32 tokens); 1024 + 1024 x 2048 gate and up, 64 tokens 24.6 / 18.5
+    (128 of 32); 5120 x 5120, 300 tokens 45.2 / 36.9 (120 of 128). With more items than SMs, 2048 x 2048: 64 tokens 18.4, in tiles of
+    32 20.5 (256); 256 tokens 37.1 and 50.0 (1024); 512 tokens in float32 30.7 and 67.6 (1024).
+    Where the pairs of SMs are all busy (``gemm_pair_sm100.cu``) they take the widest."""
+    ft, nw = (n_feat + 127) // 128, 2 if dual else 1
     wide = pick_bn(T, dual)
     n_tt = (T + wide - 1) // wide
     sk = _pick_split_k(n_tt, ft, K)
@@ -488,18 +491,10 @@ def _pick_tile(T: int, n_feat: int, K: int, dual: bool):
         sk = 1
     if T > 128 and ((T + 255) // 256) * ((nw * n_feat + 255) // 256) >= NUM_SMS // 2 and K >= 512:
         return (128 if dual else 256), sk
-    best = None
-    for bn in (32, 64, 128) if dual else (32, 64, 128, 256):
-        tiles = ((T + bn - 1) // bn) * ft
-        if bn > wide or (sk > 1 and tiles * sk * bn * nw * 128 > SPLITK_FLOATS):
-            continue
-        waves, kbs = (tiles * sk + NUM_SMS - 1) // NUM_SMS, (num_kb + sk - 1) // sk
-        main = kbs * (16384 * nw + 128 * bn * nw + 16384 * nw + 128 * bn) // 128
-        out = bn // 32 * (1400 * nw if sk == 1 else nw * (700 + 500 * sk))
-        cost = 2500 + (waves * max(main, out) + min(main, out))
-        if best is None or cost < best[0]:
-            best = (cost, bn)
-    return best[1], sk
+    for bn in (64, 128) if f32 else (32, 64, 128):
+        if bn < wide and (T + bn - 1) // bn * ft * sk <= NUM_SMS:
+            return bn, sk
+    return wide, sk
 
 
 def _pick_split_k(n_tok_tiles: int, feat_tiles: int, K: int) -> int:
@@ -682,7 +677,7 @@ def linear(x, w, residual=None, out=None, out_dtype=torch.bfloat16, split_k: Opt
         return linear_nv4(x if isinstance(x, Nv4Act) else nv4_quant_act(x), w, residual=residual, out=out)
     ws = Workspace.get(x.device)
     if bn is None and split_k is None and T > 32 and not q:
-        bn, split_k = _pick_tile(T, N, K, False)
+        bn, split_k = _pick_tile(T, N, K, False, out.dtype == torch.float32)
     bn = bn or pick_bn(T, False)
     n_tt = (T + bn - 1) // bn
     ft = (N + 127) // 128

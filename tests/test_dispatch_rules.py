@@ -22,6 +22,19 @@ def test_prompt_attention_takes_the_faster_kernel(longest, others, rows, cached,
     assert sm100.attn_on_pairs(longest + others * rows, 1 + others, longest, ctx, heads, dk) is pairs
 
 
+# tokens, features, K, gate and up, float32 -> token tile, where both sides were measured
+@pytest.mark.parametrize("T,n,K,dual,f32,bn", [
+    (128, 512, 2048, False, False, 32), (64, 1024, 2048, True, False, 32), (256, 768, 768, False, False, 32),
+    (300, 5120, 5120, False, False, 128), (130, 6176, 2048, True, False, 64),
+    (64, 2048, 2048, False, False, 64), (256, 2048, 2048, False, False, 256), (512, 2048, 2048, False, True, 256),
+    (512, 3072, 1024, False, True, 256), (64, 768, 768, False, True, 64), (96, 12352, 2048, False, False, 128),
+    (217, 1024, 2048, True, False, 128), (1024, 3072, 1024, False, False, 256), (4096, 5120, 5120, False, False, 256)])
+def test_short_prompt_products_take_the_faster_tile(T, n, K, dual, f32, bn):
+    got, sk = sm100._pick_tile(T, n, K, dual, f32)
+    wide = sm100.pick_bn(T, dual)
+    assert got == bn and sk == sm100._pick_split_k(-(-T // wide), -(-n // 128), K)
+
+
 # a batch without rows, rows that are fewer than the longest portion said to be there, one sequence of no rows beside a long one
 @pytest.mark.parametrize("T,n,longest,ctx", [(0, 1, 0, 0), (10, 1, 4096, 64), (4096, 2, 4096, 4096)])
 def test_prompt_attention_rule_takes_any_sizes(T, n, longest, ctx):
