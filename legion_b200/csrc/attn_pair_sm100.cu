@@ -2,11 +2,10 @@
 //
 // A pair of CTAs takes 256 query rows of one (sequence, query head), 128 each, and 128 keys at a time: each CTA fetches half
 // of the keys and half of the value columns, and the products of both read both halves. A CTA by itself, with 64 keys at
-// a time, moves twice the keys and values per row and reads its queries from shared memory twice as often: at head size 256
-// that is 192 KB through shared memory per 64 keys, 1500 cycles for 1024 cycles of products, and its four softmax warps
-// waited for one another's steps most of the time. 4096 tokens, single CTAs / pairs: 40 heads of 128 542 / 645 TFLOP/s, 32
-// heads of 192 (values 128) 354 / 743, before the row sums joined in the order of 64-key blocks. Bound now by the softmax (exponentials and its chain of
-// tensor-memory and barrier latencies), not by the products.
+// a time, moves twice the keys and values per row and reads its queries from shared memory twice as often, and its four
+// softmax warps wait for one another's steps most of the time. 4096 tokens, single CTAs / pairs: 40 heads of 128 over 8 key heads 318 /
+// 277 us (540 / 620 TFLOP/s), 32 heads of 192 (values 128) 486 / 232 us (354 / 740). Bound by the softmax (exponentials
+// and its chain of tensor-memory and barrier latencies), not by the products. Where it wins: attn_on_pairs in ops/sm100.py.
 //   warp 0, lane 0   TMA: queries and keys (both CTAs' copies are counted on the first CTA's barriers)
 //   warp 10, lane 0  TMA: values
 //   warp 1, lane 0   of the first CTA: all products; S(i + 1) = Q K^T is issued ahead of the softmax of block i, in the other of
@@ -41,8 +40,7 @@ struct PairAttnCfg {
   static constexpr int Q_BYTES = HALVES * 128 * 128;
   static constexpr int K_BYTES = HALVES * 64 * 128;          // 64 of the block's keys
   static constexpr int V_BYTES = VH * BKV * 128;             // half of the value columns of all its keys
-  static constexpr int VS = DV == 256 ? 3 : 4;
-  static constexpr int KS = (222 * 1024 - Q_BYTES - VS * V_BYTES) / K_BYTES >= 4 ? 4 : (DK == 256 && DV == 256 ? 2 : 3);
+  static constexpr int KS = 4, VS = 4;                       // blocks in flight
   static constexpr int RING = Q_BYTES + KS * K_BYTES + VS * V_BYTES;
   static constexpr int SMEM = RING + (2 * 2 + 1) * 128 * 4 + 512;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
@@ -295,7 +293,9 @@ pair_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         asm volatile("bar.arrive 2, 256;" ::: "memory");
       }
       alpha = 1.f;
-      // the reference moves as it would over blocks of 64 keys, so that the probabilities are rounded as the single CTA's are
+      // the reference moves as it would over blocks of 64 keys, and the sums are added in that order. Not the single CTA's bits where the
+      // second 64 keys raise the reference: the first ones' probabilities are rounded against the later one here, and against
+      // their own (and rescaled) there; either way an error of 2^-9 each
       auto follow = [&](float half) {
         const float h = half * a.scale_log2;
         if (h > m + RESCALE_LOG2 || (m == -INFINITY && h != -INFINITY)) {
@@ -446,9 +446,8 @@ int start(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, c
 int pair_attn_launch(const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const int* cu_q, const int* ctx_lens,
                      const int* block_table, int table_width, int page, int n_seqs, int max_q_len, int Hq, int Hkv, int dk,
                      int dv, float scale_log2, void* out, int* status, cudaStream_t s) {
-  // head sizes above 192 stay on single CTAs: a maximum that grows by more than 2^8 in the second 64 keys of a block rounds the
-  // first ones' probabilities anew, and models with 4-bit activations turn that into 3% of their outputs after 32768 tokens
-  // (this path was twice as fast there)
+  // head sizes above 192 stay on single CTAs: the rounding against a later reference (above) becomes 3% of the outputs of models
+  // with 4-bit activations after 32768 tokens, and those are the ones with such heads (pairs were twice as fast there)
   if (64 % page || dk <= 64 || dv <= 64 || dk > 192 || dv > 128 || (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
   PairAttnArgs a{cu_q, ctx_lens, block_table, table_width, page, Hq, Hkv, scale_log2, static_cast<__nv_bfloat16*>(out), dk, dv,
                  status};

@@ -118,6 +118,9 @@ struct WgemmHost {
 };
 
 int wgemm_launch(const WgemmHost& h, cudaStream_t stream);
+// the kernel on pairs of SMs (gemm_pair_sm100.cu): whether it takes this launch, and its start (0: started, else *err)
+bool wgemm_pair_ok(const WgemmHost& h, const WgemmArgs& a, int sms);
+int wgemm_pair_launch(const WgemmHost& h, const WgemmArgs& a, int sms, cudaStream_t stream, const char** err);
 int wgemm_pick_bn(int n_tok_per_tile_hint, bool dual);
 size_t wgemm_workspace_floats(int bn, bool dual, int n_tok_tiles, int feat_tiles, int split_k);
 const char* wgemm_last_error();
