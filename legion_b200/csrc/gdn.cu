@@ -250,8 +250,9 @@ int gdn_recurrent_launch(const void* qkv, long ld, const float* g, const float* 
 // CTA is rewriting. Every sequence contributes exactly one token (row `seq` of proj).
 // Bound by the state, read and written once (2 x 2 MB per sequence for 32 heads of 128 x 128), as long as it stays in
 // registers: a thread holds DK / NS cells of one column. Two value heads take 1024 threads of 32 cells; 512 threads of 64
-// cells, compiled for blocks of up to 1024, had 64 registers and spilled: 64 / 16 / 1 sequences took 94 / 24 / 11 us, now
-// 66 / 17 / 7 (42 us is what the state of 64 takes at 6.46 TB/s).
+// cells, compiled for blocks of up to 1024, had 64 registers and spilled: 64 / 16 / 1 sequences took 86 / 29 / 16 us, now
+// 74 / 25 / 12 (single launches behind a flush of L2, of which some 5 us are none of the kernel's; 42 us is what the state of 64
+// takes at 6.46 TB/s). The odd threads go on from the even ones' sums, two barriers more in the chain.
 //   proj row = [q (Hk*DK) | k (Hk*DK) | v (Hv*DV) | z (Hv*DV) | b (Hv) | a (Hv)]  (the fused input projection)
 // Intermediate values are rounded to bf16 where the separate kernels store them as bf16 (conv outputs, the
 // recurrence output), so a decode step gives the same numbers as the multi-kernel path used for verify rows.
@@ -384,7 +385,9 @@ int gdn_decode_fused_launch(const void* proj, long ld, const float* conv_w, floa
   if (Hk <= 0 || Hv % Hk || Hv / Hk > 4 || KC != 4) return 1;
   const int r = Hv / Hk;
   dim3 grid(Hk, n_seqs);
-  // threads per column of a head: four where a block of all the key head's value heads has room for them, else two
+  // threads per column of a head: four where a block of all the key head's value heads has room for them, else two. At 64 columns
+  // three and four value heads take two as well: with four, 1024 threads of 16 cells, 64 sequences of 32 heads (4 per key head)
+  // took 33 us against 25
 #define LB_GF(D_, R_, NS_, THREADS_)                                                                                \
   if (DK == D_ && DV == D_ && r <= R_) {                                                                            \
     launch_pdl(gdn_decode_fused_kernel<D_, D_, 4, NS_, THREADS_>, grid, dim3(NS_ * D_ * r), 0, s,                   \
@@ -392,7 +395,7 @@ int gdn_decode_fused_launch(const void* proj, long ld, const float* conv_w, floa
                slots, Hk, Hv, tiled_heads, scale, l2_eps, static_cast<__nv_bfloat16*>(out));                        \
     return cudaGetLastError() != cudaSuccess;                                                                       \
   }
-  LB_GF(128, 1, 4, 512) LB_GF(128, 2, 4, 1024) LB_GF(128, 4, 2, 1024) LB_GF(64, 2, 4, 512) LB_GF(64, 4, 4, 1024)
+  LB_GF(128, 1, 4, 512) LB_GF(128, 2, 4, 1024) LB_GF(128, 4, 2, 1024) LB_GF(64, 2, 4, 512) LB_GF(64, 4, 2, 1024)
 #undef LB_GF
   return 1;
 }

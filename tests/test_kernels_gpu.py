@@ -622,7 +622,7 @@ def test_fp8_gate_up_and_experts():
                                                 (300, 4, 64, 128, 128, 128)])
 def test_head_linear_in_place_slices(T, nh, K, xcol, rpg, nf):
     """Per-head projections through one grouped GEMM launch: each head's activation slice is read in place (column
-    offset in the TMA coordinate) and its output rows go through the row map."""
+    offset in the TMA coordinate) and its output rows lie between those of the other heads."""
     torch.manual_seed(T)
     x = rnd(T, nh * xcol)
     w = rnd(nh * rpg, K, scale=0.1)
@@ -638,7 +638,8 @@ def test_head_linear_in_place_slices(T, nh, K, xcol, rpg, nf):
 
 
 @pytest.mark.parametrize("nk,nv,d,tiled,n_seq", [(2, 4, 128, False, 5), (4, 8, 64, True, 16), (2, 2, 128, False, 1),
-                                                (16, 32, 128, False, 3)])
+                                                (16, 32, 128, False, 3), (2, 6, 64, False, 3), (3, 12, 64, True, 2),
+                                                (2, 2, 64, False, 2), (1, 3, 128, True, 2), (2, 8, 128, False, 2)])
 def test_gdn_decode_fused_matches_the_separate_kernels(nk, nv, d, tiled, n_seq):
     """One launch (conv + gates + delta rule + gated norm) against the four-kernel path and the fp32 reference,
     outputs and both carried states, over two consecutive decode steps."""
