@@ -478,9 +478,10 @@ def _pick_tile(T: int, n_feat: int, K: int, dual: bool, f32: bool = False):
     and with them the 4-bit activations behind them, do not depend on the tile. With the widest tile short prompts ran on
     a few SMs, whose last CTAs added up to nine partial sums of 256 tokens each: the tile is the narrowest with which all work
     items still run at once, else the widest (more items than SMs repeat the weights' way through shared memory and the
-    partial sums' way through memory). float32 rows leave 32-token tiles one element at a time: 64 at least.
+    partial sums' way through memory). Where the widest tile's items leave two SMs in five without work, some rounds of a tile a
+    quarter as wide or less still pay. float32 rows leave 32-token tiles one element at a time: 64 at least.
     Widest / this, us: 512 x 2048, 128 tokens 26.6 / 14.4 (128 items of 32 tokens); 1024 + 1024 x 2048 gate and up, 64 tokens 24.6 / 18.5
-    (128 of 32); 5120 x 5120, 300 tokens 45.2 / 36.9 (120 of 128). With more items than SMs, 2048 x 2048: 64 tokens 18.4, in tiles of
+    (128 of 32); 5120 x 5120, 300 tokens 45.2 / 36.9 (120 of 128); 576 x 4096, 217 tokens 63.5 / 52.3 (560 of 32). With more items than SMs, 2048 x 2048: 64 tokens 18.4, in tiles of
     32 20.5 (256); 256 tokens 37.1 and 50.0 (1024); 512 tokens in float32 30.7 and 67.6 (1024).
     Where the pairs of SMs are all busy (``gemm_pair_sm100.cu``) they take the widest."""
     ft, nw = (n_feat + 127) // 128, 2 if dual else 1
@@ -491,8 +492,10 @@ def _pick_tile(T: int, n_feat: int, K: int, dual: bool, f32: bool = False):
         sk = 1
     if T > 128 and ((T + 255) // 256) * ((nw * n_feat + 255) // 256) >= NUM_SMS // 2 and K >= 512:
         return (128 if dual else 256), sk
+    idle = sk > 1 and not f32 and n_tt * ft * sk <= NUM_SMS * 3 // 5
     for bn in (64, 128) if f32 else (32, 64, 128):
-        if bn < wide and (T + bn - 1) // bn * ft * sk <= NUM_SMS:
+        rounds = 0.625 * (wide // bn) if idle and wide >= 4 * bn else 1
+        if bn < wide and (T + bn - 1) // bn * ft * sk <= NUM_SMS * rounds:
             return bn, sk
     return wide, sk
 

@@ -28,7 +28,8 @@ def test_prompt_attention_takes_the_faster_kernel(longest, others, rows, cached,
     (300, 5120, 5120, False, False, 128), (130, 6176, 2048, True, False, 64),
     (64, 2048, 2048, False, False, 64), (256, 2048, 2048, False, False, 256), (512, 2048, 2048, False, True, 256),
     (512, 3072, 1024, False, True, 256), (64, 768, 768, False, True, 64), (96, 12352, 2048, False, False, 128),
-    (217, 1024, 2048, True, False, 128), (1024, 3072, 1024, False, False, 256), (4096, 5120, 5120, False, False, 256)])
+    (256, 576, 4096, False, False, 32), (384, 576, 4096, False, False, 256), (96, 576, 4096, False, False, 32), (48, 576, 4096, False, False, 64),
+    (130, 3072, 1024, False, False, 256), (217, 1024, 2048, True, False, 128), (1024, 3072, 1024, False, False, 256), (4096, 5120, 5120, False, False, 256)])
 def test_short_prompt_products_take_the_faster_tile(T, n, K, dual, f32, bn):
     got, sk = sm100._pick_tile(T, n, K, dual, f32)
     wide = sm100.pick_bn(T, dual)
